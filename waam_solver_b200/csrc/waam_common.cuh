@@ -230,6 +230,10 @@ struct VarPhase {
 // kernels.py:1686-1707 lookup_table_1d: clamped to the end knots, linear
 // inside; where knots repeat, the last segment containing T wins.  Every
 // index is a compile-time constant, so the knots stay in parameter space.
+// The segment is chosen first and divided once: a division per segment (up to
+// 28 for a cell's four properties) made the refresh, not memory, the bound
+// of the table path's thermal stage (131x67x50: 52.5 -> 29.4 us with its
+// register limit, waam_fused.cu k_thermal_list).
 __device__ __forceinline__ float table_lookup(float T, const float (&t)[WAAM_TABLE_KNOTS],
                                               const float (&v)[WAAM_TABLE_KNOTS], int n,
                                               float fallback) {
@@ -248,15 +252,21 @@ __device__ __forceinline__ float table_lookup(float T, const float (&t)[WAAM_TAB
         } else if (T >= t_last) {
             result = v_last;
         } else {
+            float t0 = 0.0f, t1 = 0.0f, v0 = 0.0f, v1 = 0.0f;
+            bool inside = false;
 #pragma unroll
             for (int idx = 0; idx < WAAM_TABLE_KNOTS - 1; ++idx) {
-                if (idx < n - 1) {
-                    const float t0 = t[idx], t1 = t[idx + 1];
-                    if (T >= t0 && T <= t1) {
-                        const float w = (T - t0) / (t1 - t0 + 1e-8f);
-                        result = v[idx] + w * (v[idx + 1] - v[idx]);
-                    }
+                if (idx < n - 1 && T >= t[idx] && T <= t[idx + 1]) {
+                    t0 = t[idx];
+                    t1 = t[idx + 1];
+                    v0 = v[idx];
+                    v1 = v[idx + 1];
+                    inside = true;
                 }
+            }
+            if (inside) {
+                const float w = (T - t0) / (t1 - t0 + 1e-8f);
+                result = v0 + w * (v1 - v0);
             }
         }
     }

@@ -858,9 +858,10 @@ __global__ void __launch_bounds__(256) k_thermal_fused(
 // step already left both enthalpy / temperature buffers equal there and its
 // column pass left f_l = 0 (GAS): the stage would rewrite the same values.
 // Six blocks per SM without tables (at most 42 registers; measured: the stage
-// 22 % faster); the table form keeps its registers.
+// 22 % faster), five with them (48 registers): left to itself the compiler
+// took 204 registers for the table form, one block per SM.
 template <bool TABLES>
-__global__ void __launch_bounds__(256, TABLES ? 1 : 6) k_thermal_list(
+__global__ void __launch_bounds__(256, TABLES ? 5 : 6) k_thermal_list(
     Dims d, const float* __restrict__ H, float* __restrict__ H_next, const float* __restrict__ T,
     float* __restrict__ T_next, float* __restrict__ f_l, const float* __restrict__ ux,
     const float* __restrict__ uy, const float* __restrict__ uz, const int32_t* __restrict__ flags,
