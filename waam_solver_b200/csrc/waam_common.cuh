@@ -1071,7 +1071,62 @@ __device__ __forceinline__ void collide_mrt_cell(const float* f, float fl, float
 #undef WAAM_FEQ
 }
 
-// kernels.py:2778-2885 collide_srt for one cell
+// a * ex(q) + b * ey(q) + c * ez(q) without the products: a factor of one is
+// the value itself, and for finite a, b, c a factor of zero adds a zero.
+template <int Q>
+__device__ __forceinline__ float along(float a, float b, float c) {
+    float s = ex(Q) == 1 ? a : (ex(Q) == -1 ? -a : 0.0f);
+    if (ey(Q) != 0) {
+        const float t = ey(Q) == 1 ? b : -b;
+        s = ex(Q) != 0 ? s + t : t;
+    }
+    if (ez(Q) != 0) {
+        const float t = ez(Q) == 1 ? c : -c;
+        s = ex(Q) != 0 || ey(Q) != 0 ? s + t : t;
+    }
+    return s;
+}
+
+// The population update of collide_srt with every product written out: cells
+// with an infinity or a NaN, whose products with zero are NaN.
+static __device__ __noinline__ void srt_update_nonfinite(const float* f, float fl, float fx,
+                                                         float fy, float fz, float omega,
+                                                         float C_darcy, float* out, float* mom) {
+    const float eps = 1e-6f;
+    float r = 0.0f, jx = 0.0f, jy = 0.0f, jz = 0.0f;
+    for (int q = 0; q < 19; ++q) {
+        const float fq = f[q];
+        r += fq;
+        jx += fq * (float)ex(q);
+        jy += fq * (float)ey(q);
+        jz += fq * (float)ez(q);
+    }
+    const float inv_r = 1.0f / (r + eps);
+    const float om = 1.0f - fl;
+    const float ck = 1.0f + C_darcy * (om * om) / (fl * fl * fl + eps);
+    const float u = (jx * inv_r + 0.5f * fx * inv_r) / ck;
+    const float v = (jy * inv_r + 0.5f * fy * inv_r) / ck;
+    const float w = (jz * inv_r + 0.5f * fz * inv_r) / ck;
+    const float u2 = u * u + v * v + w * w;
+    for (int q = 0; q < 19; ++q) {
+        const float eu = (float)ex(q) * u + (float)ey(q) * v + (float)ez(q) * w;
+        const float feq = wq(q) * r * (1.0f + 3.0f * eu + 4.5f * eu * eu - 1.5f * u2);
+        const float Fe = (float)ex(q) * fx + (float)ey(q) * fy + (float)ez(q) * fz;
+        const float S = wq(q) * (1.0f - 0.5f * omega) *
+                        (3.0f * Fe + 9.0f * (eu * Fe) - 3.0f * (u * fx + v * fy + w * fz));
+        out[q] = f[q] - omega * (f[q] - feq) + S;
+    }
+    mom[0] = r;
+    mom[1] = u;
+    mom[2] = v;
+    mom[3] = w;
+}
+
+// kernels.py:2778-2885 collide_srt for one cell.  The reference multiplies by
+// the lattice vectors' components (-1, 0, 1), 12 products per population;
+// for finite values they only choose terms, so they are chosen at compile
+// time (about 400 instructions instead of 900; the same bits up to the sign
+// of a zero).  A cell that is not finite takes the written-out form.
 __device__ __forceinline__ void collide_srt_cell(const float* f, float fl, float fx, float fy,
                                                  float fz, float omega, float C_darcy, float* out,
                                                  float& r, float& u, float& v, float& w) {
@@ -1080,11 +1135,11 @@ __device__ __forceinline__ void collide_srt_cell(const float* f, float fl, float
     float jx = 0.0f, jy = 0.0f, jz = 0.0f;
 #pragma unroll
     for (int q = 0; q < 19; ++q) {
-        float fq = f[q];
+        const float fq = f[q];
         r += fq;
-        jx += fq * (float)ex(q);
-        jy += fq * (float)ey(q);
-        jz += fq * (float)ez(q);
+        if (ex(q) != 0) jx = ex(q) == 1 ? jx + fq : jx - fq;
+        if (ey(q) != 0) jy = ey(q) == 1 ? jy + fq : jy - fq;
+        if (ez(q) != 0) jz = ez(q) == 1 ? jz + fq : jz - fq;
     }
     float inv_r = 1.0f / (r + eps);
     float uxr = jx * inv_r + 0.5f * fx * inv_r;
@@ -1095,17 +1150,32 @@ __device__ __forceinline__ void collide_srt_cell(const float* f, float fl, float
     u = uxr / ck;
     v = uyr / ck;
     w = uzr / ck;
-    float u2 = u * u + v * v + w * w;
-#pragma unroll
-    for (int q = 0; q < 19; ++q) {
-        float eu = (float)ex(q) * u + (float)ey(q) * v + (float)ez(q) * w;
-        float wqq = wq(q);
-        float feq = wqq * r * (1.0f + 3.0f * eu + 4.5f * eu * eu - 1.5f * u2);
-        float Fe = (float)ex(q) * fx + (float)ey(q) * fy + (float)ez(q) * fz;
-        float S = wqq * (1.0f - 0.5f * omega) *
-                  (3.0f * Fe + 9.0f * (eu * Fe) - 3.0f * (u * fx + v * fy + w * fz));
-        out[q] = f[q] - omega * (f[q] - feq) + S;
+    if (!(isfinite(r) && isfinite(u) && isfinite(v) && isfinite(w) && isfinite(fx) &&
+          isfinite(fy) && isfinite(fz))) {
+        float g[19], og[19], m[4];
+        for (int q = 0; q < 19; ++q) g[q] = f[q];
+        srt_update_nonfinite(g, fl, fx, fy, fz, omega, C_darcy, og, m);
+        for (int q = 0; q < 19; ++q) out[q] = og[q];
+        r = m[0];
+        u = m[1];
+        v = m[2];
+        w = m[3];
+        return;
     }
+    const float u2 = u * u + v * v + w * w;
+    const float uF = 3.0f * (u * fx + v * fy + w * fz);
+    const float pre = 1.0f - 0.5f * omega;
+#define WAAM_SRT(Q)                                                                     \
+    {                                                                                   \
+        const float eu = along<Q>(u, v, w), Fe = along<Q>(fx, fy, fz);                  \
+        const float feq = wq(Q) * r * (1.0f + 3.0f * eu + 4.5f * eu * eu - 1.5f * u2);  \
+        const float S = wq(Q) * pre * (3.0f * Fe + 9.0f * (eu * Fe) - uF);              \
+        out[Q] = f[Q] - omega * (f[Q] - feq) + S;                                       \
+    }
+    WAAM_SRT(0) WAAM_SRT(1) WAAM_SRT(2) WAAM_SRT(3) WAAM_SRT(4) WAAM_SRT(5) WAAM_SRT(6)
+    WAAM_SRT(7) WAAM_SRT(8) WAAM_SRT(9) WAAM_SRT(10) WAAM_SRT(11) WAAM_SRT(12) WAAM_SRT(13)
+    WAAM_SRT(14) WAAM_SRT(15) WAAM_SRT(16) WAAM_SRT(17) WAAM_SRT(18)
+#undef WAAM_SRT
 }
 
 // kernels.py:3312-3335 clamp_velocity_mach for one cell
