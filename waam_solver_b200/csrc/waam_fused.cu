@@ -186,17 +186,20 @@ int launch_contact_columns(Dims d, const float* snap, float* phi, const int32_t*
 
 // ---------------------------------------------------------------------------
 // Pull streaming (kernels.py:2971-3010): x periodic, y/z clamped, bounce-back
-// from SOLID sources for non-gas cells.  Every thread first issues its 19
-// source loads back to back (independent addresses, so all are in flight at
-// once), then, for the few non-gas cells, replaces the populations whose
-// source is SOLID by the cell's own opposite population, then stores.
-// The per-population base pointers come precomputed in the launch
-// parameters -- for interior cells (no wrap or clamp on any axis) already
-// shifted by the pull offset -- so an address costs one multiply-add.
+// from SOLID sources for non-gas cells.  Threads take consecutive cells of the
+// whole grid, so no lane is lost where nz is not a multiple of 32, and a
+// warp's row and the next one, whose sectors the k-shifted pulls share, run
+// in one block.  The pull offset of population q is the same for every cell
+// but for the faces, where the wrap or the clamp adds a distance per axis
+// (StreamShift, zero inside): no cell takes a path of its own.  Every thread
+// first issues its 19 source loads back to back (independent addresses, so
+// all are in flight at once), then, for the non-gas cells, replaces the
+// populations whose source is SOLID by the cell's own opposite population,
+// then stores.
 // ---------------------------------------------------------------------------
 template <typename T>
 struct StreamPtrs {
-    const T* src[19];    // population q shifted by the interior pull offset
+    const T* src[19];    // population q of the input, shifted by the pull offset
     const T* base[19];   // population q of the input
     T* dst[19];          // population q of the output
 };
@@ -207,7 +210,7 @@ static StreamPtrs<T> stream_ptrs(const Dims& d, const void* f_src, void* f_dst) 
     const int64_t n = d.n(), sx = (int64_t)d.ny * d.nz, sy = d.nz;
     const uintptr_t a = reinterpret_cast<uintptr_t>(f_src), b = reinterpret_cast<uintptr_t>(f_dst);
     for (int q = 0; q < 19; ++q) {
-        const int64_t off = ex(q) * sx + ey(q) * sy + ez(q);   // < n for every q >= 1, 0 for q = 0
+        const int64_t off = ex(q) * sx + ey(q) * sy + ez(q);
         P.src[q] = reinterpret_cast<const T*>(a + (uintptr_t)((q * n - off) * (int64_t)sizeof(T)));
         P.base[q] = reinterpret_cast<const T*>(a + (uintptr_t)(q * n * (int64_t)sizeof(T)));
         P.dst[q] = reinterpret_cast<T*>(b + (uintptr_t)(q * n * (int64_t)sizeof(T)));
@@ -215,69 +218,214 @@ static StreamPtrs<T> stream_ptrs(const Dims& d, const void* f_src, void* f_dst) 
     return P;
 }
 
-__device__ __forceinline__ int stream_source(const Dims& d, bool interior, int i, int j, int k,
-                                             int c, int q) {
-    if (interior) return c - (ex(q) * d.ny * d.nz + ey(q) * d.nz + ez(q));
-    int ni = i - ex(q);
-    ni = ni < 0 ? ni + d.nx : (ni >= d.nx ? ni - d.nx : ni);
-    const int nj = imax(0, imin(j - ey(q), d.ny - 1));
-    const int nk = imax(0, imin(k - ez(q), d.nz - 1));
-    return (ni * d.ny + nj) * d.nz + nk;
+// Division by a fixed divisor for every 32-bit dividend (Granlund and
+// Montgomery, "Division by invariant integers using multiplication", PLDI
+// 1994, figure 4.1): q = (((x - t) >> s1) + t) >> s2, t = high word of m x.
+struct FastDiv {
+    unsigned m, s1, s2;
+    static FastDiv of(unsigned divisor) {
+        unsigned l = 0;
+        while ((1ull << l) < divisor) ++l;
+        FastDiv f;
+        f.m = (unsigned)(((1ull << 32) * ((1ull << l) - divisor)) / divisor + 1);
+        f.s1 = l < 1 ? l : 1;
+        f.s2 = l < 1 ? 0 : l - 1;
+        return f;
+    }
+    __device__ __forceinline__ unsigned div(unsigned x) const {
+        const unsigned t = __umulhi(m, x);
+        return (((x - t) >> s1) + t) >> s2;
+    }
+};
+
+struct StreamGrid {
+    int n, nz, sx;       // cells; cells of a column; of an x plane
+    int nx, ny;
+    FastDiv by_nz, by_ny;
+};
+
+// What the wrap and the clamps add to the pull offset of a cell: [0] for
+// populations moving down an axis (e = -1, pulled from above), [2] up.
+struct StreamShift {
+    int x[3], y[3], z[3];
+    template <int Q>
+    __device__ __forceinline__ int of() const {
+        int s = 0;
+        if (ex(Q) != 0) s += x[ex(Q) + 1];
+        if (ey(Q) != 0) s += y[ey(Q) + 1];
+        if (ez(Q) != 0) s += z[ez(Q) + 1];
+        return s;
+    }
+};
+
+__device__ __forceinline__ StreamShift stream_shift(const StreamGrid& g, int c, int& k) {
+    const unsigned r = g.by_nz.div((unsigned)c);
+    k = c - (int)r * g.nz;
+    const unsigned i = g.by_ny.div(r);
+    const int j = (int)r - (int)i * g.ny;
+    StreamShift s;
+    s.x[0] = (int)i == g.nx - 1 ? -g.n : 0;
+    s.x[2] = i == 0u ? g.n : 0;
+    s.y[0] = j == g.ny - 1 ? -g.nz : 0;
+    s.y[2] = j == 0 ? g.nz : 0;
+    s.z[0] = k == g.nz - 1 ? -1 : 0;
+    s.z[2] = k == 0 ? 1 : 0;
+    return s;
 }
 
-// T is the stored element: streaming moves stored values unchanged, whatever
-// the population storage.
+// The bounce-back of one streamed non-gas cell, after the stream's stores.
 template <typename T>
-__device__ __forceinline__ void stream_cell(const Dims& d, const StreamPtrs<T>& P,
-                                            const int32_t* __restrict__ flags, int i, int j,
-                                            int k, int c) {
-    const int flag = flags[c];
-    if (flag == SOLID) return;
-    const bool interior = i > 0 && i < d.nx - 1 && j > 0 && j < d.ny - 1 && k > 0 && k < d.nz - 1;
-    T v[19];
-    if (interior) {
+__device__ __noinline__ void bounce_cell(const StreamGrid& g, const StreamPtrs<T>& P,
+                                         const int32_t* flags, int c) {
+    int k;
+    const StreamShift s = stream_shift(g, c, k);
+    unsigned back = 0u;
+#define WAAM_SRC(Q) (c - (ex(Q) * g.sx + ey(Q) * g.nz + ez(Q)) + s.of<Q>())
+#define WAAM_BACK(Q) back |= flags[WAAM_SRC(Q)] == SOLID ? 1u << Q : 0u;
+    WAAM_BACK(1) WAAM_BACK(2) WAAM_BACK(3) WAAM_BACK(4) WAAM_BACK(5) WAAM_BACK(6)
+    WAAM_BACK(7) WAAM_BACK(8) WAAM_BACK(9) WAAM_BACK(10) WAAM_BACK(11) WAAM_BACK(12)
+    WAAM_BACK(13) WAAM_BACK(14) WAAM_BACK(15) WAAM_BACK(16) WAAM_BACK(17) WAAM_BACK(18)
+#undef WAAM_BACK
+#undef WAAM_SRC
 #pragma unroll
-        for (int q = 0; q < 19; ++q) v[q] = P.src[q][c];
-    } else {
-#pragma unroll
-        for (int q = 0; q < 19; ++q) v[q] = P.base[q][stream_source(d, false, i, j, k, c, q)];
-    }
-    if (flag != GAS) {
-#pragma unroll
-        for (int q = 1; q < 19; ++q)
-            if (flags[stream_source(d, interior, i, j, k, c, q)] == SOLID) v[q] = P.base[opp(q)][c];
-    }
-#pragma unroll
-    for (int q = 0; q < 19; ++q) P.dst[q][c] = v[q];
+    for (int q = 1; q < 19; ++q)
+        if ((back >> q) & 1u) P.dst[q][c] = P.base[opp(q)][c];
 }
 
 __device__ __forceinline__ bool is_active(int flag) { return flag == FLUID || flag == IFACE; }
 
+// T is the stored element: streaming moves stored values unchanged, whatever
+// the population storage.  Two forms, for what their grids hold:
+// VOTE, the operator: any number of fluid cells; each warp votes on the SOLID
+// cells around it.  192x96x66 all fluid: 44.8 us against 64 with a flag load
+// per population (and 32-cell rows, a third of whose lanes nz = 66 left idle).
+// Else, the fused step: few cells bounce (the melt surface), so they are
+// mended after the stores and the kernel keeps the registers of a plain copy:
+// it runs beside the step's other kernels, and what a 256x128x96 step waits
+// for is its end (0.2149 ms per step; 0.2175 with the votes' 48 registers).
 // next_flags (null: none): the flags of the step after the streamed one.
 // Cells active there (FLUID / IFACE) are left alone: that step's collision
 // writes all 19 populations of each of them into the buffer the stream
 // writes, and nothing reads that buffer between the two (the lagged stream
 // of WaamStepParams.hold_stream).
-template <typename T>
-__global__ void __launch_bounds__(256) k_stream(Dims d, const __grid_constant__ StreamPtrs<T> P,
-                                                const int32_t* __restrict__ flags,
-                                                const int32_t* __restrict__ next_flags) {
-    int i, j, k, c;
-    if (!tile_cell(d, i, j, k, c)) return;
-    if (next_flags != nullptr && is_active(next_flags[c])) return;
-    stream_cell(d, P, flags, i, j, k, c);
+constexpr int kStreamThreads = 256;
+template <typename T, bool VOTE>
+__global__ void __launch_bounds__(kStreamThreads, VOTE ? 5 : 6)
+    k_stream(const __grid_constant__ StreamGrid g, const __grid_constant__ StreamPtrs<T> P,
+             const int32_t* __restrict__ flags, const int32_t* __restrict__ next_flags) {
+    const unsigned at = blockIdx.x * kStreamThreads + threadIdx.x;
+    const bool in = at < (unsigned)g.n;
+    const int c = in ? (int)at : g.n - 1;
+    const int flag = flags[c];
+    bool work = in && flag != SOLID;
+    if (!VOTE && next_flags != nullptr) work = work && !is_active(next_flags[c]);
+    int k;
+    const StreamShift s = stream_shift(g, c, k);
+    // warps without a cell on a face skip the shifts' additions
+    const int face = s.x[0] | s.x[2] | s.y[0] | s.y[2] | s.z[0] | s.z[2];
+    const bool inside = !__any_sync(0xffffffffu, work && face != 0);
+    T v[19];
+    if (work) {
+        if (inside) {
+#pragma unroll
+            for (int q = 0; q < 19; ++q) v[q] = P.src[q][c];
+        } else {
+#define WAAM_PULL(Q) v[Q] = P.src[Q][(int64_t)c + s.of<Q>()];
+            WAAM_PULL(0) WAAM_PULL(1) WAAM_PULL(2) WAAM_PULL(3) WAAM_PULL(4) WAAM_PULL(5)
+            WAAM_PULL(6) WAAM_PULL(7) WAAM_PULL(8) WAAM_PULL(9) WAAM_PULL(10) WAAM_PULL(11)
+            WAAM_PULL(12) WAAM_PULL(13) WAAM_PULL(14) WAAM_PULL(15) WAAM_PULL(16)
+            WAAM_PULL(17) WAAM_PULL(18)
+#undef WAAM_PULL
+        }
+    }
+    if (!VOTE) {
+        if (!work) return;
+#pragma unroll
+        for (int q = 0; q < 19; ++q) P.dst[q][c] = v[q];
+        if (flag != GAS) bounce_cell(g, P, flags, c);
+        return;
+    }
+    const bool fluid = work && flag != GAS;
+    if (__any_sync(0xffffffffu, fluid)) {
+        // The SOLID sources, by warp votes: bit l of col[m] tells whether the
+        // cell beside lane l's in column (di, dj) is SOLID; a source one cell
+        // up or down is the next lane's (a clamped one the lane's own), and
+        // the end lanes load theirs.  14 flag loads in place of 18, all
+        // independent, and none of the tests where no cell is near a wall.
+        const int lane = threadIdx.x & 31;
+        unsigned col[9], any = 0u;
+        bool sol[9];
+#pragma unroll
+        for (int m = 0; m < 9; ++m) {
+            const int di = m / 3 - 1, dj = m % 3 - 1;   // pulled from (i + di, j + dj)
+            int o = c + di * g.sx + dj * g.nz;
+            if (di != 0) o += s.x[1 - di];
+            if (dj != 0) o += s.y[1 - dj];
+            sol[m] = flags[o] == SOLID;
+        }
+        unsigned end = 0u;   // the end lanes' cells below (lane 0) / above (lane 31)
+        if (lane == 0 || lane == 31) {
+            const int dk = lane == 0 ? (k > 0 ? -1 : 0) : (k < g.nz - 1 ? 1 : 0);
+#pragma unroll
+            for (int m = 1; m < 9; ++m) {
+                const int di = m / 3 - 1, dj = m % 3 - 1;
+                if (di != 0 && dj != 0) continue;
+                int o = c + di * g.sx + dj * g.nz + dk;
+                if (di != 0) o += s.x[1 - di];
+                if (dj != 0) o += s.y[1 - dj];
+                end |= flags[o] == SOLID ? 1u << m : 0u;
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < 9; ++m) {
+            col[m] = __ballot_sync(0xffffffffu, sol[m]);
+            any |= col[m];
+        }
+        if ((any != 0u || end != 0u) && fluid) {
+            const bool bot = k == 0, top = k == g.nz - 1;
+#define WAAM_BOUNCE(Q)                                                                       \
+    {                                                                                        \
+        constexpr int m = (1 - ex(Q)) * 3 + 1 - ey(Q);                                       \
+        bool b;                                                                              \
+        if (ez(Q) == 0)                                                                      \
+            b = (col[m] >> lane) & 1u;                                                       \
+        else if (ez(Q) > 0)                                                                  \
+            b = bot ? (col[m] >> lane) & 1u : ((lane == 0 ? end >> m : col[m] >> ((lane - 1) & 31)) & 1u); \
+        else                                                                                 \
+            b = top ? (col[m] >> lane) & 1u : ((lane == 31 ? end >> m : col[m] >> ((lane + 1) & 31)) & 1u); \
+        if (b) v[Q] = P.base[opp(Q)][c];                                                     \
+    }
+            WAAM_BOUNCE(1) WAAM_BOUNCE(2) WAAM_BOUNCE(3) WAAM_BOUNCE(4) WAAM_BOUNCE(5)
+            WAAM_BOUNCE(6) WAAM_BOUNCE(7) WAAM_BOUNCE(8) WAAM_BOUNCE(9) WAAM_BOUNCE(10)
+            WAAM_BOUNCE(11) WAAM_BOUNCE(12) WAAM_BOUNCE(13) WAAM_BOUNCE(14) WAAM_BOUNCE(15)
+            WAAM_BOUNCE(16) WAAM_BOUNCE(17) WAAM_BOUNCE(18)
+#undef WAAM_BOUNCE
+        }
+    }
+    if (work) {
+#pragma unroll
+        for (int q = 0; q < 19; ++q) P.dst[q][c] = v[q];
+    }
 }
 
-
-template <typename T>
+template <typename T, bool VOTE>
 static void launch_stream_t(const Dims& d, const void* f_src, void* f_dst, const int32_t* flags,
                             const int32_t* next_flags, cudaStream_t s) {
-    k_stream<T><<<tile_grid(d), tile_block(), 0, s>>>(d, stream_ptrs<T>(d, f_src, f_dst), flags,
-                                                       next_flags);
+    StreamGrid g;
+    g.n = (int)d.n();
+    g.nz = d.nz;
+    g.sx = d.ny * d.nz;
+    g.nx = d.nx;
+    g.ny = d.ny;
+    g.by_nz = FastDiv::of((unsigned)d.nz);
+    g.by_ny = FastDiv::of((unsigned)d.ny);
+    const unsigned blocks = ((unsigned)g.n + kStreamThreads - 1) / kStreamThreads;
+    k_stream<T, VOTE><<<blocks, kStreamThreads, 0, s>>>(g, stream_ptrs<T>(d, f_src, f_dst), flags,
+                                                        next_flags);
 }
 
 int launch_stream(Dims d, const float* f_src, float* f_dst, const int32_t* flags, void* stream) {
-    launch_stream_t<float>(d, f_src, f_dst, flags, nullptr, STREAM(stream));
+    launch_stream_t<float, true>(d, f_src, f_dst, flags, nullptr, STREAM(stream));
     return check_launch("k_stream");
 }
 
@@ -286,9 +434,9 @@ static int launch_stream_stored(Dims d, const void* f_src, void* f_dst, const in
                                 int storage, cudaStream_t s,
                                 const int32_t* next_flags = nullptr) {
     if (storage == kStoreF32)
-        launch_stream_t<float>(d, f_src, f_dst, flags, next_flags, s);
+        launch_stream_t<float, false>(d, f_src, f_dst, flags, next_flags, s);
     else
-        launch_stream_t<uint16_t>(d, f_src, f_dst, flags, next_flags, s);
+        launch_stream_t<uint16_t, false>(d, f_src, f_dst, flags, next_flags, s);
     return check_launch("k_stream");
 }
 
