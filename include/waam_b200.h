@@ -905,6 +905,18 @@ int waam_adj_thermal(const WaamStepParams* p, const float* lam_H, float* lam_Hp,
 int waam_adj_inject(const WaamStepParams* p, float* lam_H, const float* lam_Hp, const float* H,
                     const float* f_l, const int32_t* flags, const float* scalars, int nx, int ny,
                     int nz, double* sums, void* workspace, size_t workspace_bytes, void* stream);
+#define WAAM_MAX_COPY_PLANES 32
+/* One array of a copy: `bytes` (a multiple of 4) from src to dst, both device
+ * memory on 4-byte boundaries, not overlapping. */
+typedef struct WaamCopyPlane {
+    void* dst;
+    const void* src;
+    int64_t bytes;
+} WaamCopyPlane;
+/* Copies every listed array in one launch (the step records and checkpoints
+ * of the adjoint).  `planes` is a host array (n_planes <=
+ * WAAM_MAX_COPY_PLANES); the copies run in no particular order. */
+int waam_copy_planes(const WaamCopyPlane* planes, int n_planes, void* stream);
 /* lam[cells[t]] += vals[t] for t < count (in order) */
 int waam_adj_scatter_add(float* lam, const int32_t* cells, const float* vals, int count,
                          void* stream);

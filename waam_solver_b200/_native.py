@@ -87,6 +87,13 @@ class WaamExportChannel(C.Structure):
                 ("src", C.c_void_p * 3)]
 
 
+MAX_COPY_PLANES = 32
+
+
+class WaamCopyPlane(C.Structure):
+    _fields_ = [("dst", C.c_void_p), ("src", C.c_void_p), ("bytes", C.c_int64)]
+
+
 def _params_fields():
     """Field list of WaamStepParams, parsed from the header."""
     src = open(HEADER).read()
@@ -116,7 +123,7 @@ _CTYPES = {
     "const WaamStepParams*": C.POINTER(WaamStepParams), "const char*": C.c_char_p,
     "void* const*": C.c_void_p, "const WaamMaterialTables*": C.POINTER(WaamMaterialTables),
     "WaamTelemetry*": C.c_void_p, "const WaamProbeSet*": C.POINTER(WaamProbeSet),
-    "const WaamShiftPlane*": C.c_void_p, "const WaamExportChannel*": C.c_void_p,
+    "const WaamShiftPlane*": C.c_void_p, "const WaamCopyPlane*": C.c_void_p, "const WaamExportChannel*": C.c_void_p,
     "double*": C.c_void_p, "uint8_t*": C.c_void_p, "const uint8_t*": C.c_void_p,
     "int64_t*": C.c_void_p, "unsigned long long*": C.c_void_p,
 }

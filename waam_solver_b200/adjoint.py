@@ -49,15 +49,31 @@ def _stream():
     return torch.cuda.current_stream().cuda_stream
 
 
+def _copy_planes(pairs):
+    """dst <- src for every (dst, src) pair of contiguous tensors, in one launch
+    (per 32 of them)."""
+    for s0 in range(0, len(pairs), _native.MAX_COPY_PLANES):
+        part = pairs[s0:s0 + _native.MAX_COPY_PLANES]
+        table = (_native.WaamCopyPlane * len(part))()
+        for row, (dst, src) in zip(table, part):
+            row.dst, row.src = dst.data_ptr(), src.data_ptr()
+            row.bytes = src.numel() * src.element_size()
+        _call("waam_copy_planes", ctypes.byref(table), len(part), _stream())
+
+
+def _state_tensors(g):
+    return [getattr(g, k) for k in _FIELDS] + list(g._H) + list(g._T)
+
+
 class _Checkpoint:
     """Device copy of the full twin state (every field a step reads or writes)."""
 
     def __init__(self, tw):
         g = tw.grid
         g.flush_stream()
-        self.t = {k: getattr(g, k).clone() for k in _FIELDS}
-        self.t["_H"] = [h.clone() for h in g._H]
-        self.t["_T"] = [x.clone() for x in g._T]
+        state = _state_tensors(g)
+        self.t = [torch.empty_like(t) for t in state]
+        _copy_planes(list(zip(self.t, state)))
         self.g_host = (g._read_buf is g.f_a, g._cur, getattr(g, "_forces_dirty", True),
                        getattr(g, "_tracers_live", False))
         self.host = {k: getattr(tw, k) for k in _HOST}
@@ -68,12 +84,7 @@ class _Checkpoint:
         g._collide_pending = False
         g._lag_pending = False
         g._tiles_valid = False          # the quiet-tile history is not the checkpoint's
-        for k in _FIELDS:
-            getattr(g, k).copy_(self.t[k])
-        for dst, src in zip(g._H, self.t["_H"]):
-            dst.copy_(src)
-        for dst, src in zip(g._T, self.t["_T"]):
-            dst.copy_(src)
+        _copy_planes(list(zip(_state_tensors(g), self.t)))
         read_a, g._cur, g._forces_dirty, live = self.g_host
         g._read_buf, g._write_buf = (g.f_a, g.f_b) if read_a else (g.f_b, g.f_a)
         if live != getattr(g, "_tracers_live", False):
@@ -102,6 +113,13 @@ class _Tape:
         self.tf = torch.empty((K, 19, cap), **f32)
         self.tcells = torch.empty((K, cap), dtype=torch.int32, device=dev)
         self.tcount = torch.zeros(K, dtype=torch.int32, device=dev)
+
+    def record(self, g, slot):
+        """The state after a step into its slot."""
+        _copy_planes([(self.H[slot], g.H), (self.T[slot], g.T), (self.fl[slot], g.f_l),
+                      (self.phi[slot], g.phi), (self.flags[slot], g.flags),
+                      (self.u[slot, 0], g.ux), (self.u[slot, 1], g.uy), (self.u[slot, 2], g.uz),
+                      (self.scal[slot], g.step_scalars)])
 
 
 def _grid_pre(g):
@@ -426,15 +444,7 @@ def _taped_step(tw, x, y, tape, slot):
     g.flip_thermal()
     g.swap_buffers()
     tw._step_n += 1
-    tape.H[slot].copy_(g.H.reshape(-1))
-    tape.T[slot].copy_(g.T.reshape(-1))
-    tape.fl[slot].copy_(g.f_l.reshape(-1))
-    tape.phi[slot].copy_(g.phi.reshape(-1))
-    tape.flags[slot].copy_(g.flags.reshape(-1))
-    tape.u[slot, 0].copy_(g.ux.reshape(-1))
-    tape.u[slot, 1].copy_(g.uy.reshape(-1))
-    tape.u[slot, 2].copy_(g.uz.reshape(-1))
-    tape.scal[slot].copy_(g.step_scalars)
+    tape.record(g, slot)
 
 
 class CoupledStepLoss(torch.autograd.Function):

@@ -54,13 +54,26 @@ __device__ void accumulate_sums(double (&v)[NR], Workspace ws, double* out) {
     __syncthreads();
     if (!last) return;
     __threadfence();
+    // every thread adds a fixed strided subset of each sum's partials, then the
+    // same tree as above: the order never changes (one thread adding 592
+    // partials one after another took most of the kernel's time; with it and
+    // the 32-bit cell decode, 128x64x48: inject 31.6 -> 18 us, mu 30.6 -> 11)
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+        v[r] = 0.0;
+        for (unsigned b = threadIdx.x; b < gridDim.x; b += kAdjThreads)
+            v[r] += __ldcg(ws.partials + (int64_t)r * gridDim.x + b);
+        for (int o = 16; o > 0; o >>= 1) v[r] += __shfl_down_sync(0xffffffffu, v[r], o);
+    }
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+        for (int r = 0; r < NR; ++r) sh[r][warp] = v[r];
+    __syncthreads();
     if (threadIdx.x < NR) {
-        const volatile double* part = ws.partials;
         double t = 0.0;
-        for (unsigned b = 0; b < gridDim.x; ++b) t += part[(int64_t)threadIdx.x * gridDim.x + b];
+        for (int w = 0; w < kAdjThreads / 32; ++w) t += sh[threadIdx.x][w];
         out[threadIdx.x] += t;
     }
-    __syncthreads();
     if (threadIdx.x == 0) *ws.counter = 0u;
 }
 
@@ -79,44 +92,83 @@ __device__ __forceinline__ void cell_ijk(const Dims& d, int64_t c, int& i, int& 
 // clamp(j - e_y) = j_s, clamp(k - e_z) = k_s: one cell, plus the cell itself
 // on a clamped y / z face.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_adj_stream(Dims d, float* __restrict__ lam_yp,
-                                                    const float* __restrict__ lam_xp,
-                                                    float* __restrict__ lam_xn,
-                                                    const int32_t* __restrict__ flags) {
-    int i, j, k, s;
-    if (!tile_cell(d, i, j, k, s)) return;
+// One source cell per thread, consecutive cells of the whole grid.  Population
+// q has the destination s + off(q) and, on a y / z face, up to three clamped
+// ones beside it (every row has face cells, so they take the common path, not
+// one of their own: a warp with a serial loop over its few face cells held the
+// kernel at 60 us on 128x64x48; 56 us with 32-cell rows, 41 us now).  The destinations' flags are turned into bit
+// sets first, so that all population loads of a cell are independent, and
+// every load comes before any store (the compiler cannot know that the 19
+// planes of lam_yp are distinct).
+__global__ void __launch_bounds__(256, 3) k_adj_stream(Dims d, CellDecode dec,
+                                                       float* __restrict__ lam_yp,
+                                                       const float* __restrict__ lam_xp,
+                                                       float* __restrict__ lam_xn,
+                                                       const int32_t* __restrict__ flags) {
+    const unsigned at = blockIdx.x * 256u + threadIdx.x;
+    if (at >= (unsigned)d.n()) return;
+    const int s = (int)at;
+    int i, j, k;
+    dec.ijk(s, i, j, k);
     const int64_t n = d.n();
+    const int sx = d.ny * d.nz, sy = d.nz;
     const int fs = flags[s];
+    const bool solid = fs == SOLID, own = fs != GAS && !solid;   // own: may have bounced
+    const int east = i == d.nx - 1 ? sx - (int)n : sx, west = i == 0 ? (int)n - sx : -sx;
+    const bool south = j == 0, north = j == d.ny - 1, bot = k == 0, top = k == d.nz - 1;
+    auto xoff = [&](int q) { return ex(q) == 1 ? east : (ex(q) == -1 ? west : 0); };
+    auto j_in = [&](int q) { return !((ey(q) == 1 && north) || (ey(q) == -1 && south)); };
+    auto k_in = [&](int q) { return !((ez(q) == 1 && top) || (ez(q) == -1 && bot)); };
+    // a clamped pull: the cell on the face also takes from its own row / level
+    auto j_too = [&](int q) { return (ey(q) == 1 && south) || (ey(q) == -1 && north); };
+    auto k_too = [&](int q) { return (ez(q) == 1 && bot) || (ez(q) == -1 && top); };
+    // the cell one step along q, with y and z clamped: q's destination where
+    // in range, and the cell that opp(q) of s pulls from
+    auto step = [&](int q) {
+        return s + xoff(q) + (j_in(q) ? ey(q) * sy : 0) + (k_in(q) ? ez(q) : 0);
+    };
+    // does a cell with flag fc take population q from this one?
+    auto takes = [&](int q, int fc) { return q == 0 || !solid ? fc != SOLID : fc == GAS; };
+    unsigned take = 0u, back = 0u;
 #pragma unroll
     for (int q = 0; q < 19; ++q) {
-        float acc = lam_yp[q * n + s];
-        int ic = i + ex(q);
-        ic = ic < 0 ? ic + d.nx : (ic >= d.nx ? ic - d.nx : ic);
-        int jc[2], kc[2], nj = 0, nk = 0;
-        const int j1 = j + ey(q), k1 = k + ez(q);
-        if (j1 >= 0 && j1 < d.ny) jc[nj++] = j1;
-        if ((ey(q) == 1 && j == 0) || (ey(q) == -1 && j == d.ny - 1)) jc[nj++] = j;
-        if (k1 >= 0 && k1 < d.nz) kc[nk++] = k1;
-        if ((ez(q) == 1 && k == 0) || (ez(q) == -1 && k == d.nz - 1)) kc[nk++] = k;
-        for (int a = 0; a < nj; ++a)
-            for (int b = 0; b < nk; ++b) {
-                const int c = d.idx(ic, jc[a], kc[b]);
-                const int fc = flags[c];
-                if (fc == SOLID) continue;                      // not written by the stream
-                if (q != 0 && fc != GAS && fs == SOLID) continue;   // bounced back instead
-                acc += lam_xp[q * n + c];
-            }
-        // bounce-back: s (non-gas) took population opp(q) from its own Y'[q]
-        if (q != 0 && fs != GAS && fs != SOLID) {
-            const int qo = opp(q);
-            int ni = i - ex(qo);
-            ni = ni < 0 ? ni + d.nx : (ni >= d.nx ? ni - d.nx : ni);
-            const int nj2 = imax(0, imin(j - ey(qo), d.ny - 1));
-            const int nk2 = imax(0, imin(k - ez(qo), d.nz - 1));
-            if (flags[d.idx(ni, nj2, nk2)] == SOLID) acc += lam_xp[qo * n + s];
+        const int fc = flags[step(q)];
+        if (j_in(q) && k_in(q) && takes(q, fc)) take |= 1u << q;
+        if (q != 0 && own && fc == SOLID) back |= 1u << q;   // s took opp(q) from its own Y'[q]
+    }
+    float acc[19], x[19];
+#pragma unroll
+    for (int q = 0; q < 19; ++q) acc[q] = lam_yp[q * n + s];
+#pragma unroll
+    for (int q = 0; q < 19; ++q) x[q] = lam_xp[q * n + ((take >> q) & 1u ? step(q) : s)];
+#pragma unroll
+    for (int q = 0; q < 19; ++q)
+        if ((take >> q) & 1u) acc[q] += x[q];
+    if (south || north || bot || top) {
+#pragma unroll
+        for (int q = 1; q < 19; ++q) {
+            const int c = s + xoff(q);
+            if (ez(q) != 0 && k_too(q) && j_in(q) && takes(q, flags[c + ey(q) * sy]))
+                acc[q] += lam_xp[q * n + c + ey(q) * sy];
+            if (ey(q) != 0 && j_too(q) && k_in(q) && takes(q, flags[c + ez(q)]))
+                acc[q] += lam_xp[q * n + c + ez(q)];
+            if (ey(q) != 0 && ez(q) != 0 && j_too(q) && k_too(q) && takes(q, flags[c]))
+                acc[q] += lam_xp[q * n + c];
         }
-        lam_yp[q * n + s] = acc;
-        lam_xn[q * n + s] = fs == SOLID ? lam_xp[q * n + s] : 0.0f;
+    }
+    if (back != 0u) {
+#pragma unroll
+        for (int q = 1; q < 19; ++q)
+            if ((back >> q) & 1u) acc[q] += lam_xp[opp(q) * n + s];
+    }
+#pragma unroll
+    for (int q = 0; q < 19; ++q) lam_yp[q * n + s] = acc[q];
+    if (solid) {
+#pragma unroll
+        for (int q = 0; q < 19; ++q) lam_xn[q * n + s] = lam_xp[q * n + s];
+    } else {
+#pragma unroll
+        for (int q = 0; q < 19; ++q) lam_xn[q * n + s] = 0.0f;
     }
 }
 
@@ -353,19 +405,23 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_thermal_mu(
     float* __restrict__ lam_ux, float* __restrict__ lam_uy, float* __restrict__ lam_uz,
     const float* __restrict__ Hs, const float* __restrict__ T, const float* __restrict__ ux,
     const float* __restrict__ uy, const float* __restrict__ uz,
-    const int32_t* __restrict__ flags, AdjThermalArgs a, Workspace ws, double* grad) {
+    const int32_t* __restrict__ flags, AdjThermalArgs a, CellDecode dec, Workspace ws,
+    double* grad) {
     double sums[1] = {0.0};
-    const int64_t n = d.n();
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n;
-         c += (int64_t)gridDim.x * blockDim.x) {
+    const unsigned n = (unsigned)d.n();
+    for (unsigned at = blockIdx.x * blockDim.x + threadIdx.x; at < n;
+         at += gridDim.x * blockDim.x) {
+        const int c = (int)at;
         const int flag = flags[c];
         const float lh = lam_H[c];
-        if (flag == GAS) {
+        // a zero adjoint stays zero and has no terms (most of the grid until the
+        // misfit's influence has spread, two cells a step)
+        if (flag == GAS || lh == 0.0f) {
             mu[c] = lh;
             continue;
         }
         int i, j, k;
-        cell_ijk(d, c, i, j, k);
+        dec.ijk(c, i, j, k);
         float u = 0.0f, v = 0.0f, w = 0.0f;
         if (flag != SOLID) {
             u = ux[c];
@@ -373,7 +429,8 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_thermal_mu(
             w = uz[c];
         }
         const float hc = Hs[c];
-        float h = hc + thermal_dh(d, Hs, T, flags, u, v, w, i, j, k, flag, hc, a.cpa, a.dt_lu);
+        float h = hc + thermal_dh_offsets(d, Hs, T, flags, u, v, w, i, j, k, c, flag, hc, T[c],
+                                          a.cpa, a.dt_lu);
         float dqdT = 0.0f, dqdh = 0.0f;
         bool pass = true;
         if (a.heat_loss) {
@@ -448,7 +505,24 @@ __global__ void __launch_bounds__(256) k_adj_thermal_gather(
     if (!tile_cell(d, i, j, k, s)) return;
     float acc_h = mu[s];
     float acc_t = 0.0f;
-    const int fs = flags[s];
+    // the adjoints that can reach s: none set, nothing to gather (this and the
+    // diffusion from seven flags instead of 49: 25 -> 16 us on 128x64x48)
+    {
+        const int sx = d.ny * d.nz, sy = d.nz;
+        bool any = acc_h != 0.0f;
+#pragma unroll
+        for (int o = 1; o <= 2; ++o) {
+            const float m[6] = {i >= o ? mu[s - o * sx] : 0.0f, i + o < d.nx ? mu[s + o * sx] : 0.0f,
+                                j >= o ? mu[s - o * sy] : 0.0f, j + o < d.ny ? mu[s + o * sy] : 0.0f,
+                                k >= o ? mu[s - o] : 0.0f,      k + o < d.nz ? mu[s + o] : 0.0f};
+#pragma unroll
+            for (int q = 0; q < 6; ++q) any |= m[q] != 0.0f;
+        }
+        if (!any) {
+            lam_Hp[s] = acc_h;
+            return;
+        }
+    }
     // advection: candidates on the three axis lines through s, offsets -2..2
 #pragma unroll
     for (int ax = 0; ax < 3; ++ax) {
@@ -476,32 +550,30 @@ __global__ void __launch_bounds__(256) k_adj_thermal_gather(
             }
         }
     }
-    // diffusion: c = s (centre and fallback slots) and the six neighbours
-    {
-        const int di[7] = {0, 1, -1, 0, 0, 0, 0}, dj[7] = {0, 0, 0, 1, -1, 0, 0};
-        const int dk[7] = {0, 0, 0, 0, 0, 1, -1};
+    // diffusion.  A cell's Laplacian reads its six neighbours, a gas or missing
+    // one replaced by the cell itself: s appears in its own with -6 plus its
+    // replaced neighbours, in a neighbour's with 1 (none of it if s is gas).
+    const int fs = flags[s];
+    if (fs != GAS) {
+        const int di[6] = {1, -1, 0, 0, 0, 0}, dj[6] = {0, 0, 1, -1, 0, 0};
+        const int dk[6] = {0, 0, 0, 0, 1, -1};
+        bool use[6];
+        float m[6], cs = -6.0f;
 #pragma unroll
-        for (int m7 = 0; m7 < 7; ++m7) {
-            const int ic = i + di[m7], jc = j + dj[m7], kc = k + dk[m7];
-            if (ic < 0 || ic >= d.nx || jc < 0 || jc >= d.ny || kc < 0 || kc >= d.nz) continue;
-            const int c = d.idx(ic, jc, kc);
-            if (flags[c] == GAS) continue;
-            const float m = mu[c];
-            if (m == 0.0f) continue;
-            // c's six slots: the neighbour if in range and not gas, else c itself
-            float cs = m7 == 0 ? -6.0f : 0.0f;
-            const int nb[6] = {d.idx(imax(0, ic - 1), jc, kc), d.idx(imin(ic + 1, d.nx - 1), jc, kc),
-                               d.idx(ic, imax(0, jc - 1), kc), d.idx(ic, imin(jc + 1, d.ny - 1), kc),
-                               d.idx(ic, jc, imax(0, kc - 1)), d.idx(ic, jc, imin(kc + 1, d.nz - 1))};
-#pragma unroll
-            for (int sl = 0; sl < 6; ++sl) {
-                const int src = flags[nb[sl]] == GAS ? c : nb[sl];
-                if (src == s) cs += 1.0f;
-            }
-            if (cs != 0.0f) acc_t += m * cpa * dt_lu * cs;
+        for (int q = 0; q < 6; ++q) {
+            const int ic = i + di[q], jc = j + dj[q], kc = k + dk[q];
+            const bool in = ic >= 0 && ic < d.nx && jc >= 0 && jc < d.ny && kc >= 0 && kc < d.nz;
+            const int c = in ? d.idx(ic, jc, kc) : s;
+            use[q] = in && flags[c] != GAS;
+            m[q] = use[q] ? mu[c] : 0.0f;
+            if (!use[q]) cs += 1.0f;
         }
+        const float m0 = mu[s];
+        if (m0 != 0.0f && cs != 0.0f) acc_t += m0 * cpa * dt_lu * cs;
+#pragma unroll
+        for (int q = 0; q < 6; ++q)
+            if (m[q] != 0.0f) acc_t += m[q] * cpa * dt_lu;
     }
-    (void)fs;
     lam_Hp[s] = acc_h;
     if (acc_t != 0.0f) lam_T[s] += acc_t;
 }
@@ -519,18 +591,19 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_inject(
     Dims d, float* __restrict__ lam_H, const float* __restrict__ lam_Hp,
     const float* __restrict__ H, const float* __restrict__ f_l,
     const int32_t* __restrict__ flags, const float* __restrict__ scalars, ArcParams p,
-    float arc_k_offset, float sigma, int welding, int cap, PhaseParams ph, Workspace ws,
-    double* sums_out) {
+    float arc_k_offset, float sigma, int welding, int cap, PhaseParams ph, CellDecode dec,
+    Workspace ws, double* sums_out) {
     double sums[kInjectSums];
 #pragma unroll
     for (int r = 0; r < kInjectSums; ++r) sums[r] = 0.0;
-    const int64_t n = d.n();
+    const unsigned n = (unsigned)d.n();
     p.arc_k = scalars[kScalarArcK] + arc_k_offset;
     p.arc_i = scalars[kScalarArcI];
     p.arc_j = scalars[kScalarArcJ];
     const float epw = scalars[kScalarEpw];
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n;
-         c += (int64_t)gridDim.x * blockDim.x) {
+    for (unsigned at = blockIdx.x * blockDim.x + threadIdx.x; at < n;
+         at += gridDim.x * blockDim.x) {
+        const int c = (int)at;
         const float lh = lam_Hp[c];
         const int flag = flags[c];
         if (!welding || flag == GAS) {
@@ -538,7 +611,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_inject(
             continue;
         }
         int i, j, k;
-        cell_ijk(d, c, i, j, k);
+        dec.ijk(c, i, j, k);
         const float fl = f_l[c];
         const float wd = arc_weight(k, p.arc_k, fl, p.pen, p.enable);
         const bool weighted = !(wd < 1e-6f);
@@ -564,11 +637,9 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_inject(
 #pragma unroll
             for (int q = 0; q < 5; ++q) sums[6 + q] += (double)(wd * dw[q]);
         }
-        float dh = 0.0f;
-        bool hit = false;
-        if (epw > 0.0f && weighted) {
-            hit = arc_cell_heat(p, epw, i, j, k, flag, fl, dh);
-        }
+        // arc_cell_heat (waam_common.cuh) with the weight found above
+        const bool hit = epw > 0.0f && weighted;
+        const float dh = hit ? epw * w * wd : 0.0f;
         float h = H[c];
         if (hit) h = h + dh;
         bool pass = true;
@@ -590,10 +661,67 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_inject(
     accumulate_sums<kInjectSums>(sums, ws, sums_out);
 }
 
-// lam[cells[t]] += vals[t], one thread in order (a handful of probe cells).
+// lam[cells[t]] += vals[t] in order, one warp: of the lanes of 32 entries that
+// name one cell the first adds their values one after another, so a cell that
+// is named twice sums as the loop over t would.
 __global__ void k_adj_scatter_add(float* lam, const int32_t* cells, const float* vals, int count) {
-    if (blockIdx.x == 0 && threadIdx.x == 0)
-        for (int t = 0; t < count; ++t) lam[cells[t]] += vals[t];
+    const int lane = threadIdx.x;
+    for (int t0 = 0; t0 < count; t0 += 32) {
+        const int t = t0 + lane;
+        const bool in = t < count;
+        const int cell = in ? cells[t] : -1;
+        const float v = in ? vals[t] : 0.0f;
+        const unsigned same = __match_any_sync(0xffffffffu, cell);
+        const bool first = in && __ffs(same) - 1 == lane;
+        float acc = first ? lam[cell] : 0.0f;
+        for (int o = 0; o < 32; ++o) {
+            const float w = __shfl_sync(0xffffffffu, v, o);
+            if (first && ((same >> o) & 1u)) acc += w;
+        }
+        if (first) lam[cell] = acc;
+        __syncwarp();
+    }
+}
+
+// Many arrays in one launch.  A block copies kCopyBytes of one array; the
+// blocks of array p are first[p] .. first[p + 1] - 1.  16 bytes per access
+// where the array and its copy are aligned to them, else 4.  (A 128x64x48
+// step's record is ten arrays of 1.6 MB: ten copy calls took 25 us of the
+// device and 60 us of the host.)
+constexpr int kCopyThreads = 256;
+constexpr int64_t kCopyBytes = kCopyThreads * 16 * 4;
+struct CopyTable {
+    WaamCopyPlane p[WAAM_MAX_COPY_PLANES];
+    unsigned first[WAAM_MAX_COPY_PLANES + 1];
+    int n;
+};
+
+__global__ void __launch_bounds__(kCopyThreads) k_copy_planes(const __grid_constant__ CopyTable T) {
+    int p = 0;
+    while (p + 1 < T.n && blockIdx.x >= T.first[p + 1]) ++p;
+    const int64_t at = (int64_t)(blockIdx.x - T.first[p]) * kCopyBytes;
+    const int64_t bytes = T.p[p].bytes - at < kCopyBytes ? T.p[p].bytes - at : kCopyBytes;
+    char* dst = static_cast<char*>(T.p[p].dst) + at;
+    const char* src = static_cast<const char*>(T.p[p].src) + at;
+    const bool wide = ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15) == 0;
+    int64_t done = 0;
+    if (wide) {
+        const int64_t n16 = bytes / 16;
+        uint4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int64_t e = u * kCopyThreads + threadIdx.x;
+            if (e < n16) v[u] = reinterpret_cast<const uint4*>(src)[e];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int64_t e = u * kCopyThreads + threadIdx.x;
+            if (e < n16) reinterpret_cast<uint4*>(dst)[e] = v[u];
+        }
+        done = n16 * 16;
+    }
+    for (int64_t e = done / 4 + threadIdx.x; e < bytes / 4; e += kCopyThreads)
+        reinterpret_cast<uint32_t*>(dst)[e] = reinterpret_cast<const uint32_t*>(src)[e];
 }
 
 AdjThermalArgs thermal_args(const WaamStepParams* p) {
@@ -631,8 +759,9 @@ int waam_adj_stream(float* lam_yp, const float* lam_xp, float* lam_xn, const int
     REQUIRE(lam_yp && lam_xp && lam_xn && flags, "adj_stream: null field");
     REQUIRE(lam_yp != lam_xp && lam_xn != lam_xp && lam_xn != lam_yp, "adj_stream: aliasing");
     Dims d{nx, ny, nz};
-    k_adj_stream<<<tile_grid(d), tile_block(), 0, STREAM(stream)>>>(d, lam_yp, lam_xp, lam_xn,
-                                                                     flags);
+    const unsigned blocks = ((unsigned)d.n() + 255u) / 256u;
+    k_adj_stream<<<blocks, 256, 0, STREAM(stream)>>>(d, CellDecode::of(d), lam_yp, lam_xp, lam_xn,
+                                                     flags);
     return check_launch("k_adj_stream");
 }
 
@@ -708,7 +837,8 @@ int waam_adj_thermal(const WaamStepParams* p, const float* lam_H, float* lam_Hp,
     AdjThermalArgs a = thermal_args(p);
     Workspace ws = Workspace::at(workspace);
     k_adj_thermal_mu<<<kAdjBlocks, kAdjThreads, 0, STREAM(stream)>>>(
-        d, lam_H, mu, lam_T, lam_ux, lam_uy, lam_uz, Hp, T, ux, uy, uz, flags, a, ws, grad_hconv);
+        d, lam_H, mu, lam_T, lam_ux, lam_uy, lam_uz, Hp, T, ux, uy, uz, flags, a, CellDecode::of(d),
+        ws, grad_hconv);
     int e = check_launch("k_adj_thermal_mu");
     if (e) return e;
     k_adj_thermal_gather<<<tile_grid(d), tile_block(), 0, STREAM(stream)>>>(
@@ -739,8 +869,31 @@ int waam_adj_inject(const WaamStepParams* p, float* lam_H, const float* lam_Hp, 
     PhaseParams ph = make_phase(p->cp_rho, p->L_rho, p->Ts, p->Tl, p->T_cap, p->cap_enabled);
     k_adj_inject<<<kAdjBlocks, kAdjThreads, 0, STREAM(stream)>>>(
         d, lam_H, lam_Hp, H, f_l, flags, scalars, a, p->arc_k_offset, p->sigma_heat, p->welding,
-        p->cap_enabled, ph, Workspace::at(workspace), sums);
+        p->cap_enabled, ph, CellDecode::of(d), Workspace::at(workspace), sums);
     return check_launch("k_adj_inject");
+}
+
+int waam_copy_planes(const WaamCopyPlane* planes, int n_planes, void* stream) {
+    REQUIRE(planes && n_planes >= 0 && n_planes <= WAAM_MAX_COPY_PLANES,
+            "copy_planes: bad plane table");
+    CopyTable t;
+    t.n = 0;
+    int64_t blocks = 0;
+    for (int q = 0; q < n_planes; ++q) {
+        const WaamCopyPlane& p = planes[q];
+        REQUIRE(p.bytes >= 0 && p.bytes % 4 == 0, "copy_planes: bytes not a multiple of 4");
+        if (p.bytes == 0) continue;
+        REQUIRE(p.dst && p.src, "copy_planes: null array");
+        REQUIRE(((reinterpret_cast<uintptr_t>(p.dst) | reinterpret_cast<uintptr_t>(p.src)) & 3) == 0,
+                "copy_planes: misaligned array");
+        t.p[t.n] = p;
+        t.first[t.n++] = (unsigned)blocks;
+        blocks += (p.bytes + kCopyBytes - 1) / kCopyBytes;
+        REQUIRE(blocks <= INT32_MAX, "copy_planes: too many bytes");
+    }
+    if (t.n == 0) return WAAM_OK;
+    k_copy_planes<<<(unsigned)blocks, kCopyThreads, 0, STREAM(stream)>>>(t);
+    return check_launch("k_copy_planes");
 }
 
 int waam_adj_scatter_add(float* lam, const int32_t* cells, const float* vals, int count,

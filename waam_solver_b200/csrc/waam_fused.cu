@@ -218,26 +218,6 @@ static StreamPtrs<T> stream_ptrs(const Dims& d, const void* f_src, void* f_dst) 
     return P;
 }
 
-// Division by a fixed divisor for every 32-bit dividend (Granlund and
-// Montgomery, "Division by invariant integers using multiplication", PLDI
-// 1994, figure 4.1): q = (((x - t) >> s1) + t) >> s2, t = high word of m x.
-struct FastDiv {
-    unsigned m, s1, s2;
-    static FastDiv of(unsigned divisor) {
-        unsigned l = 0;
-        while ((1ull << l) < divisor) ++l;
-        FastDiv f;
-        f.m = (unsigned)(((1ull << 32) * ((1ull << l) - divisor)) / divisor + 1);
-        f.s1 = l < 1 ? l : 1;
-        f.s2 = l < 1 ? 0 : l - 1;
-        return f;
-    }
-    __device__ __forceinline__ unsigned div(unsigned x) const {
-        const unsigned t = __umulhi(m, x);
-        return (((x - t) >> s1) + t) >> s2;
-    }
-};
-
 struct StreamGrid {
     int n, nz, sx;       // cells; cells of a column; of an x plane
     int nx, ny;

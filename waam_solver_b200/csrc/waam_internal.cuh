@@ -60,6 +60,41 @@ __device__ __forceinline__ bool tile_cell(const Dims& d, int& i, int& j, int& k,
     return true;
 }
 
+// Division by a fixed divisor for every 32-bit dividend (Granlund and
+// Montgomery, "Division by invariant integers using multiplication", PLDI
+// 1994, figure 4.1): q = (((x - t) >> s1) + t) >> s2, t = high word of m x.
+struct FastDiv {
+    unsigned m, s1, s2;
+    static FastDiv of(unsigned divisor) {
+        unsigned l = 0;
+        while ((1ull << l) < divisor) ++l;
+        FastDiv f;
+        f.m = (unsigned)(((1ull << 32) * ((1ull << l) - divisor)) / divisor + 1);
+        f.s1 = l < 1 ? l : 1;
+        f.s2 = l < 1 ? 0 : l - 1;
+        return f;
+    }
+    __device__ __forceinline__ unsigned div(unsigned x) const {
+        const unsigned t = __umulhi(m, x);
+        return (((x - t) >> s1) + t) >> s2;
+    }
+};
+
+// The (i, j, k) of cell c by two such divisions.
+struct CellDecode {
+    FastDiv by_nz, by_ny;
+    int nz, ny;
+    static CellDecode of(const Dims& d) {
+        return CellDecode{FastDiv::of((unsigned)d.nz), FastDiv::of((unsigned)d.ny), d.nz, d.ny};
+    }
+    __device__ __forceinline__ void ijk(int c, int& i, int& j, int& k) const {
+        const unsigned r = by_nz.div((unsigned)c);
+        k = c - (int)r * nz;
+        i = (int)by_ny.div(r);
+        j = (int)r - i * ny;
+    }
+};
+
 // Tile numbering of the quiet-tile lists: t = (i * tiles_j + j / kTileJ) *
 // tiles_k + k / kTileK (WaamFields.tile_bits / tile_list).
 __host__ __device__ inline int tiles_k(const Dims& d) { return (d.nz + kTileK - 1) / kTileK; }
