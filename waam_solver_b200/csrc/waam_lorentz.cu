@@ -158,10 +158,89 @@ __global__ void k_elec_source_sum(const float* src, int64_t n, float cell_vol, f
     *ws.counter = 0u;
 }
 
+// V consecutive cells of one column per thread: 4 where nz is a multiple of
+// four (then a group never leaves its column) and every field is 16-byte
+// aligned, so that a warp's access is 512 bytes; else 1.
+template <int V>
+__device__ __forceinline__ void load_cells(const float* p, float (&o)[V]) {
+    if constexpr (V == 4) {
+        const float4 x = *reinterpret_cast<const float4*>(p);
+        o[0] = x.x, o[1] = x.y, o[2] = x.z, o[3] = x.w;
+    } else {
+        o[0] = *p;
+    }
+}
+template <int V>
+__device__ __forceinline__ void load_cells(const int32_t* p, int (&o)[V]) {
+    if constexpr (V == 4) {
+        const int4 x = *reinterpret_cast<const int4*>(p);
+        o[0] = x.x, o[1] = x.y, o[2] = x.z, o[3] = x.w;
+    } else {
+        o[0] = *p;
+    }
+}
+template <int V>
+__device__ __forceinline__ void store_cells(float* p, const float (&o)[V]) {
+    if constexpr (V == 4)
+        *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]);
+    else
+        *p = o[0];
+}
+
+template <typename... P>
+bool quads_ok(const Dims& d, const P*... p) {
+    uintptr_t bits = 0;
+    ((bits |= reinterpret_cast<uintptr_t>(p)), ...);
+    return d.nz % 4 == 0 && bits % 16 == 0;
+}
+// A warp's share of the writing kernels: 32 consecutive k of V neighbouring
+// columns, so that it stays within one material (metal below, gas above) and
+// skips the arithmetic its cells do not need, while every thread still writes
+// 16 bytes (four columns' 128 cells in a row made every warp hold metal:
+// k_elec_J 152 us on 512x256x160 instead of 125 with one cell per thread).
+struct RowGrid {
+    FastDiv by_kt, by_ny;
+    int kt, ny, nz, ncol;
+};
+inline RowGrid row_grid(const Dims& d) {
+    const int kt = (d.nz + 31) / 32;
+    return RowGrid{FastDiv::of((unsigned)kt), FastDiv::of((unsigned)d.ny), kt, d.ny, d.nz,
+                   d.nx * d.ny};
+}
+template <int V>
+inline unsigned row_blocks(const RowGrid& g) {
+    const int64_t warps = (int64_t)((g.ncol + V - 1) / V) * g.kt;
+    return (unsigned)((warps * 32 + kThreads - 1) / kThreads);
+}
+// The thread's first cell; false: none.
+template <int V>
+__device__ __forceinline__ bool row_cells(const RowGrid& g, int& i, int& j, int& k, int& c) {
+    constexpr int kLanes = 32 / V;   // lanes per column
+    const unsigned w = (blockIdx.x * kThreads + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    const unsigned cg = g.by_kt.div(w);
+    const int col = (int)cg * V + lane / kLanes;
+    k = (int)(w - cg * (unsigned)g.kt) * 32 + (lane % kLanes) * V;
+    if (col >= g.ncol || k >= g.nz) return false;
+    i = (int)g.by_ny.div((unsigned)col);
+    j = col - i * g.ny;
+    c = col * g.nz + k;
+    return true;
+}
+// x / y.  Most quotients here are of a zero (gas, grounded metal), which over a
+// positive y is that same zero.
+__device__ __forceinline__ float quotient(float x, float y) {
+    return x == 0.0f && y > 0.0f ? x : x / y;
+}
+
 // Clear + inject + normalise in two passes that read nothing: pass 1 sums
 // value * cell_vol over the slab k_min..k_max (every other cell is 0) in
 // double, fixed order; pass 2 writes value * scale everywhere, the float the
 // reference's in-place scaling leaves.
+// Pass 1: one warp per column, lanes over the slab; a column so far from the
+// arc that every exponential of it is 0 (waam_expf below -103.98) adds nothing
+// and is left out.  A fixed grid, so the order of the sum never changes.
+constexpr int kSourceBlocks = 592;
 __global__ void __launch_bounds__(kTileK* kTileJ)
     k_elec_source_fused_sum(Dims d, float arc_i, float arc_j, float arc_k, const float* arc_k_dev,
                             float sigma_cells, float inv2s2, float current, float vol_eps,
@@ -171,15 +250,17 @@ __global__ void __launch_bounds__(kTileK* kTileJ)
     source_slab(arc_k, sigma_cells, d.nz, k_min, k_max);
     double part = 0.0;
     const int ks = imax(k_min, 0), ke = imin(k_max, d.nz - 1);
-    for (int i = blockIdx.z; i < d.nx; i += gridDim.z)
-        for (int jt = blockIdx.y; jt * kTileJ < d.ny; jt += gridDim.y)
-            for (int kt = blockIdx.x; ks + kt * kTileK <= ke; kt += gridDim.x) {
-                const int k = ks + kt * kTileK + threadIdx.x, j = jt * kTileJ + threadIdx.y;
-                if (k > ke || j >= d.ny) continue;
-                const float v = elec_source_value(i, j, k, arc_i, arc_j, arc_k, inv2s2, current,
-                                                  vol_eps, k_min, k_max);
-                part += (double)(v * cell_vol);
-            }
+    const int ncol = d.nx * d.ny, lane = threadIdx.x;
+    for (int col = blockIdx.x * kTileJ + threadIdx.y; col < ncol; col += gridDim.x * kTileJ) {
+        const int i = col / d.ny, j = col - i * d.ny;
+        const float di = (float)i - arc_i, dj = (float)j - arc_j;
+        if (-(di * di + dj * dj) * inv2s2 < -104.0f) continue;
+        for (int k = ks + lane; k <= ke; k += kTileK) {
+            const float v = elec_source_value(i, j, k, arc_i, arc_j, arc_k, inv2s2, current,
+                                              vol_eps, k_min, k_max);
+            part += (double)(v * cell_vol);
+        }
+    }
     double2 tot;
     if (finish_sum2(ws, block_sum2(part, 0.0), tot)) {
         const float total = (float)tot.x;
@@ -187,19 +268,25 @@ __global__ void __launch_bounds__(kTileK* kTileJ)
     }
 }
 
-__global__ void k_elec_source_fused_write(Dims d, float* src, float arc_i, float arc_j,
-                                          float arc_k, const float* arc_k_dev, float sigma_cells,
-                                          float inv2s2, float current, float vol_eps,
-                                          Workspace ws) {
-    int i, j, k, c;
-    if (!tile_cell(d, i, j, k, c)) return;
+// Pass 2: bound by the 4 bytes a cell it writes (512x256x160: 71 -> 51 us;
+// pass 1 57 -> 42).
+template <int V>
+__global__ void __launch_bounds__(kThreads)
+    k_elec_source_fused_write(RowGrid g, float* src, float arc_i, float arc_j, float arc_k,
+                              const float* arc_k_dev, float sigma_cells, float inv2s2,
+                              float current, float vol_eps, Workspace ws) {
+    int i, j, k, at;
+    if (!row_cells<V>(g, i, j, k, at)) return;
     if (arc_k_dev) arc_k = *arc_k_dev;
     int k_min, k_max;
-    source_slab(arc_k, sigma_cells, d.nz, k_min, k_max);
+    source_slab(arc_k, sigma_cells, g.nz, k_min, k_max);
     const float s = ws.scalars[kOpScalarSourceScale];
-    const float v = elec_source_value(i, j, k, arc_i, arc_j, arc_k, inv2s2, current, vol_eps,
-                                      k_min, k_max);
-    src[c] = v * s;
+    float o[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+        o[v] = elec_source_value(i, j, k + v, arc_i, arc_j, arc_k, inv2s2, current, vol_eps, k_min,
+                                 k_max) * s;
+    store_cells<V>(src + at, o);
 }
 
 // kernels.py:1288-1301, pass 2
@@ -337,59 +424,111 @@ __device__ __forceinline__ float jacobi_cell(float pin, float sp, float sm, floa
 // other buffer after that sweep, and every later sweep writes 0 there in the
 // reference anyway.  Fixed cells then add exactly 0 to the L1 sums of every
 // sweep after the first.  counts: [0] live cells, [1] newly fixed cells,
-// [2 + b] live cells of tile block b, then (after the scan) its list offset;
-// after those the per-block live bitmaps (one word per warp) and the totals
-// of the scan's 1024-block groups.
+// [2 + b] live cells of unit b (kUnit consecutive cells), after the scan its
+// list offset; after those one live bit per cell and the totals of the scan's
+// 1024-unit groups.
 constexpr int kCntLive = 0, kCntZero = 1, kCntBlocks = 2;
 constexpr int kLiveBlocks = 148 * 8;
-constexpr int kWarpsPerTile = kTileK * kTileJ / 32;
+constexpr int kUnit = 1024, kUnitWords = kUnit / 32;
 constexpr int kScanGroup = 1024;
 
+inline int64_t live_units(const Dims& d) { return (d.n() + kUnit - 1) / kUnit; }
 inline int64_t counts_bitmap_offset(int64_t nb) { return kCntBlocks + nb; }
-inline int64_t counts_group_offset(int64_t nb) { return kCntBlocks + nb + nb * kWarpsPerTile; }
+inline int64_t counts_group_offset(int64_t nb) { return kCntBlocks + nb + nb * kUnitWords; }
 inline int64_t counts_total_len(int64_t nb) {
     return counts_group_offset(nb) + (nb + kScanGroup - 1) / kScanGroup;
 }
 
-__device__ __forceinline__ int tile_block_linear() {
-    return (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-}
-
-__global__ void __launch_bounds__(kTileK* kTileJ)
-    k_elec_prepare(Dims d, float* __restrict__ sigma, uint8_t* __restrict__ fixed,
+// sigma, the fixed-cell mask and one live bit per cell.  Bound by memory: the
+// flags and the mask are read, sigma is written everywhere; f_l is read only
+// where a group of cells holds metal (512x256x160: 152 us with one cell per
+// thread and a block vote, 50 now).  V cells per thread (see load_cells); the
+// grid covers whole units, whose bits beyond the grid are 0.
+template <int V>
+__global__ void __launch_bounds__(kThreads)
+    k_elec_prepare(Dims d, CellDecode dec, float* __restrict__ sigma, uint8_t* __restrict__ fixed,
                    float* __restrict__ phi_b, const float* __restrict__ f_l,
                    const int32_t* __restrict__ flags, float s_liq, float s_sol, int nz_solid,
                    int* __restrict__ zero_list, int* __restrict__ counts,
                    unsigned* __restrict__ bitmaps) {
-    int i, j, k, c;
-    const bool ok = tile_cell(d, i, j, k, c);
-    bool live = false, newly = false;
-    if (ok) {
-        const int fl = flags[c];
-        sigma[c] = fl == GAS ? 1e-8f : (f_l[c] > 0.55f ? s_liq : s_sol);
-        const uint8_t nf = (fl == GAS || (k <= nz_solid && fl == SOLID)) ? 1 : 0;
-        const uint8_t of = fixed[c];
-        if (nf != of) fixed[c] = nf;
-        newly = nf && !of;
-        if (newly) phi_b[c] = 0.0f;
-        live = !nf;
+    const unsigned at = (blockIdx.x * kThreads + threadIdx.x) * V;
+    const bool in = at < (unsigned)d.n();
+    const int lane = threadIdx.x & 31;
+    unsigned live = 0u, newly = 0u;
+    if (in) {
+        int fl[V];
+        load_cells<V>(flags + at, fl);
+        unsigned of = 0u;   // the mask's V bytes
+        if constexpr (V == 4)
+            of = *reinterpret_cast<const unsigned*>(fixed + at);
+        else
+            of = fixed[at];
+        bool metal = false;
+#pragma unroll
+        for (int v = 0; v < V; ++v) metal |= fl[v] != GAS;
+        float sg[V];
+        unsigned nf = 0u;
+        if (!metal) {
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                sg[v] = 1e-8f;
+                nf |= 1u << (8 * v);
+            }
+        } else {
+            float liq[V];
+            load_cells<V>(f_l + at, liq);
+            int i, j, k;
+            dec.ijk((int)at, i, j, k);
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                sg[v] = fl[v] == GAS ? 1e-8f : (liq[v] > 0.55f ? s_liq : s_sol);
+                if (fl[v] == GAS || (k + v <= nz_solid && fl[v] == SOLID))
+                    nf |= 1u << (8 * v);
+                else
+                    live |= 1u << v;
+            }
+        }
+        store_cells<V>(sigma + at, sg);
+        if (nf != of) {
+            if constexpr (V == 4)
+                *reinterpret_cast<unsigned*>(fixed + at) = nf;
+            else
+                fixed[at] = (uint8_t)nf;
+        }
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+            if (((nf >> (8 * v)) & 1u) && !((of >> (8 * v)) & 0xffu)) {
+                newly |= 1u << v;
+                phi_b[at + v] = 0.0f;
+            }
     }
-    // newly fixed cells: one atomic per warp
-    const unsigned m = __ballot_sync(0xffffffffu, newly);
-    const int lane = (threadIdx.y * blockDim.x + threadIdx.x) & 31;
-    int base = 0;
-    if (m && lane == 0) base = atomicAdd(&counts[kCntZero], __popc(m));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (newly) zero_list[base + __popc(m & ((1u << lane) - 1u))] = c;
-    const unsigned lm = __ballot_sync(0xffffffffu, live);
-    const int b = tile_block_linear();
-    if (lane == 0) bitmaps[(int64_t)b * kWarpsPerTile + ((threadIdx.y * blockDim.x) >> 5)] = lm;
-    const int nlive = __syncthreads_count(live);
-    if (threadIdx.x == 0 && threadIdx.y == 0) counts[kCntBlocks + b] = nlive;
+    // newly fixed cells: one atomic per warp that has any
+    if (__any_sync(0xffffffffu, newly != 0u)) {
+        int incl = __popc(newly);
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        int base = 0;
+        if (lane == 31) base = atomicAdd(&counts[kCntZero], incl);
+        base = __shfl_sync(0xffffffffu, base, 31) + incl - __popc(newly);
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+            if ((newly >> v) & 1u) zero_list[base++] = (int)at + v;
+    }
+    // the live bits, one word per 32 cells
+    if constexpr (V == 4) {
+        unsigned w = live << (4 * (lane & 7));
+        for (int o = 1; o < 8; o <<= 1) w |= __shfl_xor_sync(0xffffffffu, w, o);
+        if ((lane & 7) == 0) bitmaps[at >> 5] = w;
+    } else {
+        const unsigned w = __ballot_sync(0xffffffffu, live != 0u);
+        if (lane == 0) bitmaps[at >> 5] = w;
+    }
 }
 
-// Exclusive scan of the per-block live counts in two levels: each block of
-// 1024 threads scans a group of 1024 counts (coalesced) and leaves the group
+// Exclusive scan of the units' live counts in two levels: each block of 1024
+// threads counts the bits of 1024 units, scans the counts and leaves the group
 // total; k_elec_scan_groups scans the totals; k_elec_list adds both.
 __device__ __forceinline__ int block_exclusive_scan_1024(int v, int& total) {
     __shared__ int warp_sums[32];
@@ -415,9 +554,18 @@ __device__ __forceinline__ int block_exclusive_scan_1024(int v, int& total) {
     return out;
 }
 
-__global__ void __launch_bounds__(kScanGroup) k_elec_scan(int* counts, int nb, int* groups) {
-    const int b = blockIdx.x * kScanGroup + threadIdx.x;
-    const int v = b < nb ? counts[kCntBlocks + b] : 0;
+__global__ void __launch_bounds__(kScanGroup)
+    k_elec_scan(int* counts, const unsigned* __restrict__ bitmaps, int nb, int* groups) {
+    // a warp's 32 units: 32 words each, read row by row (coalesced)
+    const int lane = threadIdx.x & 31;
+    const int b0 = blockIdx.x * kScanGroup + (threadIdx.x & ~31), b = b0 + lane;
+    int v = 0;
+#pragma unroll 8
+    for (int u = 0; u < 32; ++u) {
+        const unsigned w = b0 + u < nb ? bitmaps[(int64_t)(b0 + u) * kUnitWords + lane] : 0u;
+        const int c = (int)__reduce_add_sync(0xffffffffu, (unsigned)__popc(w));
+        if (lane == u) v = c;
+    }
     int t = 0;
     const int ex = block_exclusive_scan_1024(v, t);
     if (b < nb) counts[kCntBlocks + b] = ex;
@@ -443,13 +591,11 @@ __global__ void __launch_bounds__(kScanGroup) k_elec_scan_groups(int* counts, in
     if (threadIdx.x == 0) counts[kCntLive] = running;
 }
 
-// The live list in tile-block order (a fixed order), from the blocks' bitmaps:
-// one warp per tile block (grid-stride), which leaves at once when the block
-// has no live cells.
+// The live list in cell order, from the units' bits: one warp per unit
+// (grid-stride), which leaves at once when the unit has no live cells.
 __global__ void __launch_bounds__(256)
-    k_elec_list(Dims d, const int* __restrict__ counts, const unsigned* __restrict__ bitmaps,
-                const int* __restrict__ groups, int nb, int gx, int gy,
-                int* __restrict__ live_list) {
+    k_elec_list(const int* __restrict__ counts, const unsigned* __restrict__ bitmaps,
+                const int* __restrict__ groups, int nb, int* __restrict__ live_list) {
     const int lane = threadIdx.x & 31;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < nb; b += nwarps) {
@@ -457,14 +603,12 @@ __global__ void __launch_bounds__(256)
         const int next = b + 1 < nb ? counts[kCntBlocks + b + 1] + groups[(b + 1) / kScanGroup]
                                     : counts[kCntLive];
         if (next == off) continue;
-        const int bx = b % gx, by = (b / gx) % gy, i = b / (gx * gy);
+        const unsigned mine = bitmaps[(int64_t)b * kUnitWords + lane];
         int base = off;
-        for (int w = 0; w < kWarpsPerTile; ++w) {
-            const unsigned m = bitmaps[(int64_t)b * kWarpsPerTile + w];
-            if ((m >> lane) & 1u) {
-                const int k = bx * kTileK + lane, j = by * kTileJ + w;
-                live_list[base + __popc(m & ((1u << lane) - 1u))] = (i * d.ny + j) * d.nz + k;
-            }
+        for (int w = 0; w < kUnitWords; ++w) {
+            const unsigned m = __shfl_sync(0xffffffffu, mine, w);
+            if ((m >> lane) & 1u)
+                live_list[base + __popc(m & ((1u << lane) - 1u))] = b * kUnit + w * 32 + lane;
             base += __popc(m);
         }
     }
@@ -473,7 +617,7 @@ __global__ void __launch_bounds__(256)
 // One sweep over the live list (a fixed grid: the L1 sums in a fixed order).
 template <bool L1>
 __global__ void __launch_bounds__(256)
-    k_elec_jacobi_live(Dims d, const float* __restrict__ phi_in, float* __restrict__ phi_out,
+    k_elec_jacobi_live(Dims d, CellDecode dec, const float* __restrict__ phi_in, float* __restrict__ phi_out,
                        const float* __restrict__ sigma, const float* __restrict__ src,
                        const int* __restrict__ live_list, const int* __restrict__ counts,
                        float dx, float omega_j, const float* __restrict__ arc_k_dev,
@@ -485,9 +629,8 @@ __global__ void __launch_bounds__(256)
     double dsum = 0.0, nsum = 0.0;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < cnt; t += gridDim.x * blockDim.x) {
         const int c = live_list[t];
-        const int k = c % d.nz;
-        const int r = c / d.nz;
-        const int j = r % d.ny, i = r / d.ny;
+        int i, j, k;
+        dec.ijk(c, i, j, k);
         const int ip = c + (i + 1 < d.nx ? sx : 0), im = c - (i > 0 ? sx : 0);
         const int jp = c + (j + 1 < d.ny ? sy : 0), jm = c - (j > 0 ? sy : 0);
         const int kp = c + (k + 1 < d.nz ? 1 : 0), km = c - (k > 0 ? 1 : 0);
@@ -553,27 +696,48 @@ __global__ void __launch_bounds__(kTileK* kTileJ)
     }
 }
 
-// kernels.py:1358-1383 elec_compute_J
-__global__ void k_elec_J(Dims d, float* Jx, float* Jy, float* Jz, const float* __restrict__ phi,
-                         const float* __restrict__ sigma, const int32_t* __restrict__ flags,
-                         float dx) {
+// kernels.py:1358-1383 elec_compute_J.  Bound by the 12 bytes a cell it writes
+// (most cells are gas and take zeros): 512x256x160 125 -> 114 us.
+template <int V>
+__global__ void __launch_bounds__(kThreads)
+    k_elec_J(Dims d, RowGrid g, float* __restrict__ Jx, float* __restrict__ Jy,
+             float* __restrict__ Jz, const float* __restrict__ phi,
+             const float* __restrict__ sigma, const int32_t* __restrict__ flags, float dx) {
     int i, j, k, c;
-    if (!tile_cell(d, i, j, k, c)) return;
-    if (flags[c] == GAS) {
-        Jx[c] = 0.0f;
-        Jy[c] = 0.0f;
-        Jz[c] = 0.0f;
-        return;
+    if (!row_cells<V>(g, i, j, k, c)) return;
+    int fl[V];
+    load_cells<V>(flags + c, fl);
+    bool metal = false;
+#pragma unroll
+    for (int v = 0; v < V; ++v) metal |= fl[v] != GAS;
+    float jx[V], jy[V], jz[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) jx[v] = jy[v] = jz[v] = 0.0f;
+    if (metal) {
+        const int sx = d.ny * d.nz, sy = d.nz;
+        float sg[V], own[V], xp[V], xm[V], yp[V], ym[V];
+        load_cells<V>(sigma + c, sg);
+        load_cells<V>(phi + c, own);
+        load_cells<V>(phi + c + (i + 1 < d.nx ? sx : 0), xp);
+        load_cells<V>(phi + c - (i > 0 ? sx : 0), xm);
+        load_cells<V>(phi + c + (j + 1 < d.ny ? sy : 0), yp);
+        load_cells<V>(phi + c - (j > 0 ? sy : 0), ym);
+        const float below = phi[c - (k > 0 ? 1 : 0)];
+        const float above = phi[c + V - 1 + (k + V < d.nz ? 1 : 0)];
+        const float two_dx = 2.0f * dx;
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            if (fl[v] == GAS) continue;
+            const float zp = v + 1 < V ? own[v + 1 < V ? v + 1 : v] : above;
+            const float zm = v > 0 ? own[v > 0 ? v - 1 : v] : below;
+            jx[v] = -sg[v] * quotient(xp[v] - xm[v], two_dx);
+            jy[v] = -sg[v] * quotient(yp[v] - ym[v], two_dx);
+            jz[v] = -sg[v] * quotient(zp - zm, two_dx);
+        }
     }
-    const int sx = d.ny * d.nz, sy = d.nz;
-    const float sg = sigma[c];
-    const float two_dx = 2.0f * dx;
-    const float gx = (phi[c + (i + 1 < d.nx ? sx : 0)] - phi[c - (i > 0 ? sx : 0)]) / two_dx;
-    const float gy = (phi[c + (j + 1 < d.ny ? sy : 0)] - phi[c - (j > 0 ? sy : 0)]) / two_dx;
-    const float gz = (phi[c + (k + 1 < d.nz ? 1 : 0)] - phi[c - (k > 0 ? 1 : 0)]) / two_dx;
-    Jx[c] = -sg * gx;
-    Jy[c] = -sg * gy;
-    Jz[c] = -sg * gz;
+    store_cells<V>(Jx + c, jx);
+    store_cells<V>(Jy + c, jy);
+    store_cells<V>(Jz + c, jz);
 }
 
 __device__ __forceinline__ int radial_bin(float di, float dj, float bin_dr, int n_bins,
@@ -646,20 +810,25 @@ __global__ void __launch_bounds__(32) k_elec_bin_cols(Dims d, const float* __res
     for (int b = 0; b < n_bins; ++b) out[(int64_t)b * d.nz + k] = sacc[b * 32 + lane];
 }
 
-// One warp per bin entry: lane l adds chunks l, l + 32, ... in order, then a
-// fixed shuffle tree.
-__global__ void k_elec_bin_combine(const double* __restrict__ partials, float* bins, int nz,
-                                   int n_bins, int chunks) {
-    const int64_t m = (int64_t)nz * n_bins;
-    const int lane = threadIdx.x & 31;
-    for (int64_t q = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < m;
-         q += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-        const int b = (int)(q % n_bins), k = (int)(q / n_bins);
-        double s = 0.0;
-        for (int ch = lane; ch < chunks; ch += 32) s += partials[((int64_t)ch * n_bins + b) * nz + k];
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-        if (lane == 0) bins[q] = (float)s;
+// Block (kt, b): the chunks of bin b for 32 consecutive k (coalesced); warp w
+// adds chunks w, w + 8, ... in order, then the eight warps' sums in order.
+__global__ void __launch_bounds__(256) k_elec_bin_combine(const double* __restrict__ partials,
+                                                          float* bins, int nz, int n_bins,
+                                                          int chunks) {
+    __shared__ double sh[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int k = blockIdx.x * 32 + lane, b = blockIdx.y;
+    double s = 0.0;
+    if (k < nz) {
+#pragma unroll 8
+        for (int ch = w; ch < chunks; ch += 8) s += partials[((int64_t)ch * n_bins + b) * nz + k];
     }
+    sh[w][lane] = s;
+    __syncthreads();
+    if (w != 0 || k >= nz) return;
+    double t = sh[0][lane];
+    for (int q = 1; q < 8; ++q) t += sh[q][lane];
+    bins[(int64_t)k * n_bins + b] = (float)t;
 }
 
 __global__ void k_elec_bin_store(const double* acc, float* bins, int64_t m) {
@@ -668,48 +837,58 @@ __global__ void k_elec_bin_store(const double* acc, float* bins, int64_t m) {
         bins[q] = (float)acc[q];
 }
 
-// kernels.py:1424-1435 elec_prefix_bins (float, in place)
-__global__ void k_elec_prefix(float* bins, int n_bins, int nz) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+// kernels.py:1424-1435 elec_prefix_bins (float, in place): one warp per k, the
+// bins loaded 32 at a time and added one after another through shuffles (the
+// float order of the reference).
+__global__ void __launch_bounds__(256) k_elec_prefix(float* bins, int n_bins, int nz) {
+    const int k = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (k >= nz) return;
     float a = 0.0f;
-    for (int b = 0; b < n_bins; ++b) {
-        a += bins[(int64_t)k * n_bins + b];
-        bins[(int64_t)k * n_bins + b] = a;
+    for (int b0 = 0; b0 < n_bins; b0 += 32) {
+        const bool in = b0 + lane < n_bins;
+        const float v = in ? bins[(int64_t)k * n_bins + b0 + lane] : 0.0f;
+        const int m = imin(32, n_bins - b0);
+        float mine = 0.0f;
+        for (int o = 0; o < m; ++o) {
+            a += __shfl_sync(0xffffffffu, v, o);
+            if (o == lane) mine = a;
+        }
+        if (in) bins[(int64_t)k * n_bins + b0 + lane] = mine;
     }
 }
 
-// kernels.py:1438-1475 elec_B_axisymmetric, one warp per (i, j) column with
-// lanes over k: the column's radius, bin and r * dx come once per lane, and
-// each cell takes the reference's three divisions in its order (measured on
-// 512x256x160: 9 us per step less than one thread per cell).
-__global__ void __launch_bounds__(256) k_elec_B_cols(Dims d, float* Bx, float* By, float* Bz,
-                                                     const float* __restrict__ bins, float arc_i,
-                                                     float arc_j, float dx, float bin_dr,
-                                                     float mu0, int n_bins) {
-    const int col = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (col >= d.nx * d.ny) return;
-    const int lane = threadIdx.x & 31;
-    const int i = col / d.ny, j = col - i * d.ny;
+// kernels.py:1438-1475 elec_B_axisymmetric: V cells of a column per thread,
+// which share its radius, bin and r * dx; each cell takes the reference's
+// three divisions in its order.  Bound by those divisions where current flows
+// (512x256x160: 118 us, 127 with a warp per column), else by the 12 bytes a
+// cell it writes.
+template <int V>
+__global__ void __launch_bounds__(kThreads)
+    k_elec_B_cols(RowGrid g, float* __restrict__ Bx, float* __restrict__ By,
+                  float* __restrict__ Bz, const float* __restrict__ bins, float arc_i, float arc_j,
+                  float dx, float bin_dr, float mu0, int n_bins) {
+    int i, j, k, at;
+    if (!row_cells<V>(g, i, j, k, at)) return;
     const float di = (float)i - arc_i, dj = (float)j - arc_j;
     float rc;
     const int b = radial_bin(di, dj, bin_dr, n_bins, rc);
     const bool on = rc > 1e-3f;
     const float rm = rc * dx;
     const float two_pi = 6.28318530717958647692f;
-    const int64_t c0 = (int64_t)col * d.nz;
-    for (int k = lane; k < d.nz; k += 32) {
-        float bx = 0.0f, by = 0.0f;
+    float bx[V], by[V], bz[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        bx[v] = by[v] = bz[v] = 0.0f;
         if (on) {
-            const float I = bins[(int64_t)k * n_bins + b];
-            const float Bt = mu0 * I / (two_pi * rm);
-            bx = -Bt * dj / rc;
-            by = Bt * di / rc;
+            const float I = bins[(int64_t)(k + v) * n_bins + b];
+            const float Bt = quotient(mu0 * I, two_pi * rm);
+            bx[v] = quotient(-Bt * dj, rc);
+            by[v] = quotient(Bt * di, rc);
         }
-        Bx[c0 + k] = bx;
-        By[c0 + k] = by;
-        Bz[c0 + k] = 0.0f;
     }
+    store_cells<V>(Bx + at, bx);
+    store_cells<V>(By + at, by);
+    store_cells<V>(Bz + at, bz);
 }
 
 // kernels.py:1479-1513 apply_lorentz_JxB
@@ -787,17 +966,20 @@ static int arc_source_impl(float* source, int nx, int ny, int nz, float arc_i, f
     const float eps = 1e-6f;
     const float inv2s2 = 1.0f / (2.0f * sigma_cells * sigma_cells + eps);
     const float cell_vol = dx * dx * dx;
-    // a fixed grid: the sum order does not depend on the GPU
-    dim3 grid(imin((nz + kTileK - 1) / kTileK, 4), imin((ny + kTileJ - 1) / kTileJ, 16),
-              imin(nx, 64));
-    k_elec_source_fused_sum<<<grid, tile_block(), 0, STREAM(stream)>>>(
+    k_elec_source_fused_sum<<<kSourceBlocks, tile_block(), 0, STREAM(stream)>>>(
         d, arc_i, arc_j, arc_k, arc_k_dev, sigma_cells, inv2s2, current_A, cell_vol + eps,
         cell_vol, current_A, ws);
     int rc = check_launch("k_elec_source_fused_sum");
     if (rc) return rc;
-    k_elec_source_fused_write<<<tile_grid(d), tile_block(), 0, STREAM(stream)>>>(
-        d, source, arc_i, arc_j, arc_k, arc_k_dev, sigma_cells, inv2s2, current_A,
-        cell_vol + eps, ws);
+    const RowGrid g = row_grid(d);
+    if (quads_ok(d, source))
+        k_elec_source_fused_write<4><<<row_blocks<4>(g), kThreads, 0, STREAM(stream)>>>(
+            g, source, arc_i, arc_j, arc_k, arc_k_dev, sigma_cells, inv2s2, current_A,
+            cell_vol + eps, ws);
+    else
+        k_elec_source_fused_write<1><<<row_blocks<1>(g), kThreads, 0, STREAM(stream)>>>(
+            g, source, arc_i, arc_j, arc_k, arc_k_dev, sigma_cells, inv2s2, current_A,
+            cell_vol + eps, ws);
     return check_launch("k_elec_source_fused_write");
 }
 
@@ -920,8 +1102,7 @@ int waam_elec_jacobi_chunk(float* phi_a, float* phi_b, const float* sigma, const
 
 int64_t waam_elec_counts_len(int nx, int ny, int nz) {
     if (!dims_ok(nx, ny, nz)) return 0;
-    const dim3 g = tile_grid(Dims{nx, ny, nz});
-    return counts_total_len((int64_t)g.x * g.y * g.z);
+    return counts_total_len(live_units(Dims{nx, ny, nz}));
 }
 
 int waam_elec_prepare(float* sigma, uint8_t* fixed, float* phi_b, const float* f_l,
@@ -933,26 +1114,31 @@ int waam_elec_prepare(float* sigma, uint8_t* fixed, float* phi_b, const float* f
             "elec_prepare: null field");
     REQUIRE(counts_len >= waam_elec_counts_len(nx, ny, nz), "elec_prepare: counts too short");
     Dims d{nx, ny, nz};
-    const dim3 g = tile_grid(d);
-    const int nb = (int)(g.x * g.y * g.z);
+    const int nb = (int)live_units(d);
     cudaError_t e = cudaMemsetAsync(counts, 0, kCntBlocks * sizeof(int32_t), STREAM(stream));
     if (e != cudaSuccess) return fail(WAAM_ERR_CUDA, cudaGetErrorString(e));
     unsigned* bitmaps = reinterpret_cast<unsigned*>(counts + counts_bitmap_offset(nb));
     int* groups = counts + counts_group_offset(nb);
     const int n_groups = (nb + kScanGroup - 1) / kScanGroup;
-    k_elec_prepare<<<g, tile_block(), 0, STREAM(stream)>>>(d, sigma, fixed, phi_b, f_l, flags,
-                                                           sigma_liquid, sigma_solid, nz_solid,
-                                                           zero_list, counts, bitmaps);
+    const CellDecode dec = CellDecode::of(d);
+    const unsigned cells = (unsigned)nb * kUnit;
+    if (quads_ok(d, sigma, fixed, f_l, flags))
+        k_elec_prepare<4><<<cells / (4 * kThreads), kThreads, 0, STREAM(stream)>>>(
+            d, dec, sigma, fixed, phi_b, f_l, flags, sigma_liquid, sigma_solid, nz_solid,
+            zero_list, counts, bitmaps);
+    else
+        k_elec_prepare<1><<<cells / kThreads, kThreads, 0, STREAM(stream)>>>(
+            d, dec, sigma, fixed, phi_b, f_l, flags, sigma_liquid, sigma_solid, nz_solid,
+            zero_list, counts, bitmaps);
     int rc = check_launch("k_elec_prepare");
     if (rc) return rc;
-    k_elec_scan<<<n_groups, kScanGroup, 0, STREAM(stream)>>>(counts, nb, groups);
+    k_elec_scan<<<n_groups, kScanGroup, 0, STREAM(stream)>>>(counts, bitmaps, nb, groups);
     rc = check_launch("k_elec_scan");
     if (rc) return rc;
     k_elec_scan_groups<<<1, kScanGroup, 0, STREAM(stream)>>>(counts, groups, n_groups);
     rc = check_launch("k_elec_scan_groups");
     if (rc) return rc;
-    k_elec_list<<<kLiveBlocks, 256, 0, STREAM(stream)>>>(d, counts, bitmaps, groups, nb,
-                                                         (int)g.x, (int)g.y, live_list);
+    k_elec_list<<<kLiveBlocks, 256, 0, STREAM(stream)>>>(counts, bitmaps, groups, nb, live_list);
     return check_launch("k_elec_list");
 }
 
@@ -974,16 +1160,17 @@ int waam_elec_jacobi_live(float* phi_a, float* phi_b, const float* sigma, const 
     Dims d{nx, ny, nz};
     REQUIRE(workspace_ok(workspace, workspace_bytes, d.n()),
             "elec_jacobi_live: workspace too small or misaligned");
+    const CellDecode dec = CellDecode::of(d);
     float* in = phi_a;
     float* out = phi_b;
     for (int s = 0; s < n_sweeps; ++s) {
         if (s + 1 < n_sweeps)
             k_elec_jacobi_live<false><<<kLiveBlocks, 256, 0, STREAM(stream)>>>(
-                d, in, out, sigma, source, live_list, counts, dx, omega_j, arc_k_dev,
+                d, dec, in, out, sigma, source, live_list, counts, dx, omega_j, arc_k_dev,
                 sigma_cells, nullptr, nullptr, Workspace{});
         else
             k_elec_jacobi_live<true><<<kLiveBlocks, 256, 0, STREAM(stream)>>>(
-                d, in, out, sigma, source, live_list, counts, dx, omega_j, arc_k_dev,
+                d, dec, in, out, sigma, source, live_list, counts, dx, omega_j, arc_k_dev,
                 sigma_cells, diff_buf, norm_buf, Workspace::at(workspace));
         int rc = check_launch("k_elec_jacobi_live");
         if (rc) return rc;
@@ -1017,8 +1204,13 @@ int waam_elec_compute_J(float* Jx, float* Jy, float* Jz, const float* phi, const
     REQUIRE(dims_ok(nx, ny, nz), "elec_compute_J: bad dims");
     REQUIRE(Jx && Jy && Jz && phi && sigma && flags, "elec_compute_J: null field");
     Dims d{nx, ny, nz};
-    k_elec_J<<<tile_grid(d), tile_block(), 0, STREAM(stream)>>>(d, Jx, Jy, Jz, phi, sigma, flags,
-                                                               dx);
+    const RowGrid g = row_grid(d);
+    if (quads_ok(d, Jx, Jy, Jz, phi, sigma, flags))
+        k_elec_J<4><<<row_blocks<4>(g), kThreads, 0, STREAM(stream)>>>(d, g, Jx, Jy, Jz, phi,
+                                                                      sigma, flags, dx);
+    else
+        k_elec_J<1><<<row_blocks<1>(g), kThreads, 0, STREAM(stream)>>>(d, g, Jx, Jy, Jz, phi,
+                                                                      sigma, flags, dx);
     return check_launch("k_elec_J");
 }
 
@@ -1053,7 +1245,7 @@ int waam_elec_bin_axial_current(const float* Jz, float* bins, int nx, int ny, in
                                                 n_bins, chunk);
             int rc = check_launch("k_elec_bin_cols");
             if (rc) return rc;
-            k_elec_bin_combine<<<elem_blocks(m * 32), kThreads, 0, STREAM(stream)>>>(
+            k_elec_bin_combine<<<dim3(ktiles, n_bins), 256, 0, STREAM(stream)>>>(
                 acc, bins, nz, n_bins, chunks);
             return check_launch("k_elec_bin_combine");
         }
@@ -1071,7 +1263,7 @@ int waam_elec_bin_axial_current(const float* Jz, float* bins, int nx, int ny, in
 
 int waam_elec_prefix_bins(float* bins, int n_bins, int nz, void* stream) {
     REQUIRE(bins && n_bins >= 1 && nz >= 1, "elec_prefix_bins: bad arguments");
-    k_elec_prefix<<<(nz + 127) / 128, 128, 0, STREAM(stream)>>>(bins, n_bins, nz);
+    k_elec_prefix<<<(nz + 7) / 8, 256, 0, STREAM(stream)>>>(bins, n_bins, nz);
     return check_launch("k_elec_prefix");
 }
 
@@ -1082,9 +1274,13 @@ int waam_elec_B_axisymmetric(float* Bx, float* By, float* Bz, const float* bins,
     REQUIRE(Bx && By && Bz && bins, "elec_B_axisymmetric: null field");
     REQUIRE(n_bins >= 1, "elec_B_axisymmetric: n_bins out of range");
     Dims d{nx, ny, nz};
-    const int64_t warps = (int64_t)nx * ny;
-    k_elec_B_cols<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, STREAM(stream)>>>(
-        d, Bx, By, Bz, bins, arc_i, arc_j, dx, bin_dr_cells, mu0, n_bins);
+    const RowGrid g = row_grid(d);
+    if (quads_ok(d, Bx, By, Bz))
+        k_elec_B_cols<4><<<row_blocks<4>(g), kThreads, 0, STREAM(stream)>>>(
+            g, Bx, By, Bz, bins, arc_i, arc_j, dx, bin_dr_cells, mu0, n_bins);
+    else
+        k_elec_B_cols<1><<<row_blocks<1>(g), kThreads, 0, STREAM(stream)>>>(
+            g, Bx, By, Bz, bins, arc_i, arc_j, dx, bin_dr_cells, mu0, n_bins);
     return check_launch("k_elec_B_cols");
 }
 
