@@ -173,10 +173,54 @@ def lib():
     return _lib
 
 
-def call(name: str, *args) -> int:
-    """Call entry point ``name``; raise WaamError on a non-zero status."""
-    rc = getattr(lib(), name)(*args)
+_fns = {}
+
+
+def function(name: str):
+    """The bound entry point ``name`` (the library loaded on first use)."""
+    fn = _fns.get(name)
+    if fn is None:
+        fn = _fns[name] = getattr(lib(), name)
+    return fn
+
+
+def check(name: str, rc: int) -> int:
+    """Raise WaamError with the library's message on a non-zero status."""
     if rc != 0:
         msg = lib().waam_last_error().decode(errors="replace")
         raise WaamError("%s failed (%d): %s" % (name, rc, msg))
     return rc
+
+
+def call(name: str, *args) -> int:
+    """Call entry point ``name``; raise WaamError on a non-zero status."""
+    rc = function(name)(*args)
+    return rc if rc == 0 else check(name, rc)
+
+
+def stream_handle():
+    """cudaStream_t of torch's current stream on the current device: the value
+    of ``torch.cuda.current_stream().cuda_stream`` without building the Stream
+    object, which costs as much as a kernel launch."""
+    return _raw_stream(_current_device())
+
+
+def _stream_functions():
+    import torch
+    try:
+        torch.cuda.init()
+        raw, dev = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+        raw(dev())
+        return raw, dev
+    except (AttributeError, RuntimeError, AssertionError):
+        return (lambda _: torch.cuda.current_stream().cuda_stream), (lambda: None)
+
+
+def _current_device():
+    global _raw_stream, _current_device
+    _raw_stream, _current_device = _stream_functions()
+    return _current_device()
+
+
+def _raw_stream(device):
+    return _raw_stream(device)

@@ -32,6 +32,7 @@ import torch
 from . import _native, kernels
 from ._native import WaamError
 from .coupled_step import _fields, step_params, upload_position
+from .grid import raw_field
 
 PARAMS = ("eta", "heat_loss_factor", "arc_sigma_scale", "a_front", "a_rear", "b", "c")
 _FIELDS = ("f_a", "f_b", "rho", "ux", "uy", "uz", "T_max", "f_l", "phi", "flags", "T_prev",
@@ -42,11 +43,11 @@ _HOST = ("_step_n", "_last_droplet_time", "_last_torch_pos_m", "_torch_dir_xyz",
 
 
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr())
+    """Device address of a tensor (an address is returned as it is)."""
+    return t if type(t) is int else t.data_ptr()
 
 
-def _stream():
-    return torch.cuda.current_stream().cuda_stream
+_stream = _native.stream_handle
 
 
 def _copy_planes(pairs):
@@ -114,12 +115,46 @@ class _Tape:
         self.tcells = torch.empty((K, cap), dtype=torch.int32, device=dev)
         self.tcount = torch.zeros(K, dtype=torch.int32, device=dev)
 
+        # address of slot 0 and bytes of a slot of each record
+        self._at = {k: (t.data_ptr(), t[0].numel() * t.element_size())
+                    for k, t in vars(self).items() if isinstance(t, torch.Tensor)}
+        # the taped step's fields and the record's copy table for each state of
+        # the double buffers: they hold for the grid's fields while this tape lives
+        self._fields, self._tables = {}, {}
+
+    def at(self, name, slot):
+        """Device address of a record (an index into the tensor costs more than
+        the launch it is for)."""
+        base, size = self._at[name]
+        return base + slot * size
+
+    def fields(self, g, slot):
+        """WaamFields of a taped step with its collision tape in ``slot``."""
+        key = (g._read_buf is raw_field(g, "f_a"), g._cur, getattr(g, "_flags_copy_i", 0),
+               getattr(g, "_tracers_live", False))
+        f = self._fields.get(key)
+        if f is None:
+            f = self._fields[key] = _fields(g)
+            f.tape_cap = self.cap
+        f.tape_f, f.tape_cells = self.at("tf", slot), self.at("tcells", slot)
+        f.tape_count = self.at("tcount", slot)
+        return f
+
     def record(self, g, slot):
         """The state after a step into its slot."""
-        _copy_planes([(self.H[slot], g.H), (self.T[slot], g.T), (self.fl[slot], g.f_l),
-                      (self.phi[slot], g.phi), (self.flags[slot], g.flags),
-                      (self.u[slot, 0], g.ux), (self.u[slot, 1], g.uy), (self.u[slot, 2], g.uz),
-                      (self.scal[slot], g.step_scalars)])
+        entry = self._tables.get(g._cur)
+        if entry is None:
+            src = (("H", g.H), ("T", g.T), ("fl", g.f_l), ("phi", g.phi), ("flags", g.flags),
+                   ("u", g.ux), ("u", g.uy), ("u", g.uz), ("scal", g.step_scalars))
+            rows = (_native.WaamCopyPlane * len(src))()
+            for row, (_, t) in zip(rows, src):
+                row.src, row.bytes = t.data_ptr(), t.numel() * t.element_size()
+            entry = self._tables[g._cur] = rows, [name for name, _ in src]
+        rows, names = entry
+        n3 = self._at["u"][1] // 3
+        for q, name in enumerate(names):
+            rows[q].dst = self.at(name, slot) + ((q - 5) * n3 if name == "u" else 0)
+        _call("waam_copy_planes", ctypes.byref(rows), len(rows), _stream())
 
 
 def _grid_pre(g):
@@ -223,13 +258,19 @@ class AdjointProblem:
         self.hist = torch.zeros((self.N, max(2 * P, 2)), dtype=torch.float32, device=g.device)
         self.scal = torch.zeros((self.N, 16), dtype=torch.float32, device=g.device)
         self.checkpoints = {}
+        row = _native.WaamCopyPlane(bytes=64)
+        scal_at, hist_at = self.scal.data_ptr(), self.hist.data_ptr()
+        hist_row = 4 * self.hist.shape[1]
+        probes = kernels.probe_set(self.cell_list)
         for n, (x, y) in enumerate(self.positions):
             if n % self.K == 0:
                 self.checkpoints[n] = _Checkpoint(tw)
             tw.step(x, y, True)
-            self.scal[n].copy_(g.step_scalars)
+            row.dst, row.src = scal_at + 64 * n, g.step_scalars.data_ptr()
+            _call("waam_copy_planes", ctypes.byref(row), 1, _stream())
             if P:
-                kernels.probe_sample(g.T, g.f_l, self.cell_list, self.hist[n])
+                _call("waam_probe_sample", g.T.data_ptr(), g.f_l.data_ptr(), ctypes.byref(probes),
+                      hist_at + hist_row * n, _stream())
         self.T_probe = (self.hist[:, 0:2 * P:2].double().cpu().numpy() if P
                         else np.zeros((self.N, 0)))
         self.fl_final = g.f_l.clone()
@@ -290,20 +331,20 @@ class AdjointProblem:
             _call("waam_adj_scatter_add", _ptr(lam["fl"]), _ptr(cells),
                   _ptr(torch.tensor(coef, **f32)), ny, _stream())
         tape = _Tape(g, self.K, cap)
+        dT_at, inj_at = dT_dev.data_ptr(), inj.data_ptr()
         starts = sorted(self.checkpoints)
         for s0 in reversed(starts):
             steps = list(range(s0, min(s0 + self.K, self.N)))
             pre0 = self._record_segment(s0, steps, tape)
             for n in reversed(steps):
                 slot = n - s0
-                pre = pre0 if slot == 0 else dict(
-                    H=tape.H[slot - 1], T=tape.T[slot - 1], fl=tape.fl[slot - 1],
-                    flags=tape.flags[slot - 1], u=tape.u[slot - 1])
+                pre = pre0 if slot == 0 else {k: tape.at(k, slot - 1)
+                                              for k in ("H", "T", "fl", "flags", "u")}
                 if P:
                     _call("waam_adj_scatter_add", _ptr(lam["T"]), _ptr(self.cells),
-                          _ptr(dT_dev[n]), P, _stream())
+                          dT_at + 4 * P * n, P, _stream())
                 pops = self._reverse_step(n, slot, pre, tape, lam, pops, ctb, amap, grad_h,
-                                          inj[n], ws)
+                                          inj_at + 88 * n, ws)
         torch.cuda.synchronize()
         return self._combine(grad_h.item(), inj.cpu().numpy())
 
@@ -328,27 +369,24 @@ class AdjointProblem:
         p = ctypes.byref(self._params())
         st = _stream()
         lamX, lamY, scratch = pops
+        plane = 4 * g.n_cells
+        at = lambda name: tape.at(name, slot)  # noqa: E731
+        flags, scal = at("flags"), at("scal")
+        lu, pu = _ptr(lam["u"]), _ptr(pre["u"])
+        lH, lHp, lT, lfl = (_ptr(lam[k]) for k in ("H", "Hp", "T", "fl"))
         # un-swap: lam Y' = lam X_{n+1}, lam X' = lam Y_{n+1}
-        lam_yp, lam_xp = lamX, lamY
-        _call("waam_adj_stream", _ptr(lam_yp), _ptr(lam_xp), _ptr(scratch),
-              _ptr(tape.flags[slot]), nx, ny, nz, st)
-        lam_xn = scratch
-        _call("waam_adj_collide", p, _ptr(tape.tf[slot]), _ptr(tape.tcells[slot]),
-              _ptr(tape.tcount[slot:slot + 1]), tape.cap, _ptr(tape.phi[slot]),
-              _ptr(tape.T[slot]), _ptr(tape.fl[slot]), _ptr(tape.flags[slot]),
-              _ptr(tape.scal[slot]), _ptr(lam_yp), _ptr(lam_xn), _ptr(lam["u"][0]),
-              _ptr(lam["u"][1]), _ptr(lam["u"][2]), _ptr(lam["fl"]), _ptr(lam["T"]), _ptr(ctb),
-              _ptr(amap), nx, ny, nz, st)
-        _call("waam_adj_combine", p, _ptr(lam["H"]), _ptr(lam["T"]), _ptr(lam["fl"]),
-              _ptr(tape.H[slot]), _ptr(tape.flags[slot]), _ptr(tape.phi[slot]), g.n_cells, st)
-        _call("waam_adj_thermal", p, _ptr(lam["H"]), _ptr(lam["Hp"]), _ptr(lam["mu"]),
-              _ptr(lam["T"]), _ptr(lam["u"][0]), _ptr(lam["u"][1]), _ptr(lam["u"][2]),
-              _ptr(tape.Hp[slot]), _ptr(pre["T"]), _ptr(pre["u"][0]), _ptr(pre["u"][1]),
-              _ptr(pre["u"][2]), _ptr(pre["flags"]), nx, ny, nz, _ptr(grad_h), _ptr(ws),
-              ws.numel(), st)
-        _call("waam_adj_inject", p, _ptr(lam["H"]), _ptr(lam["Hp"]), _ptr(pre["H"]),
-              _ptr(pre["fl"]), _ptr(pre["flags"]), _ptr(tape.scal[slot]), nx, ny, nz,
-              _ptr(inj_row), _ptr(ws), ws.numel(), st)
+        lam_yp, lam_xp, lam_xn = lamX, lamY, scratch
+        yp, xn = _ptr(lam_yp), _ptr(lam_xn)
+        _call("waam_adj_stream", yp, _ptr(lam_xp), xn, flags, nx, ny, nz, st)
+        _call("waam_adj_collide", p, at("tf"), at("tcells"), at("tcount"), tape.cap, at("phi"),
+              at("T"), at("fl"), flags, scal, yp, xn, lu, lu + plane, lu + 2 * plane, lfl, lT,
+              _ptr(ctb), _ptr(amap), nx, ny, nz, st)
+        _call("waam_adj_combine", p, lH, lT, lfl, at("H"), flags, at("phi"), g.n_cells, st)
+        _call("waam_adj_thermal", p, lH, lHp, _ptr(lam["mu"]), lT, lu, lu + plane, lu + 2 * plane,
+              at("Hp"), _ptr(pre["T"]), pu, pu + plane, pu + 2 * plane, _ptr(pre["flags"]), nx, ny,
+              nz, _ptr(grad_h), _ptr(ws), ws.numel(), st)
+        _call("waam_adj_inject", p, lH, lHp, _ptr(pre["H"]), _ptr(pre["fl"]), _ptr(pre["flags"]),
+              scal, nx, ny, nz, _ptr(inj_row), _ptr(ws), ws.numel(), st)
         # new (lam X_n, lam Y_n, scratch)
         return [lam_xn, lam_yp, lam_xp]
 
@@ -427,17 +465,14 @@ def _taped_step(tw, x, y, tape, slot):
     p.clear_forces = 1 if getattr(g, "_forces_dirty", True) else 0
     dx_, dy_, dz_ = tw._torch_dir_xyz
     p.dir_x, p.dir_y, p.dir_z = dx_, dy_, dz_
-    f = _fields(g)
-    f.tape_f = tape.tf[slot].data_ptr()
-    f.tape_cells = tape.tcells[slot].data_ptr()
-    f.tape_count = tape.tcount[slot:slot + 1].data_ptr()
-    f.tape_cap = tape.cap
+    f = tape.fields(g, slot)
     g._pos_dst = g.step_scalars[4:6]
     upload_position(tw, arc_i, arc_j)
     ws = g.workspace
     st = _stream()
     _native.call("waam_step_pre", ctypes.byref(f), ctypes.byref(p), ws.data_ptr(), ws.numel(), st)
-    tape.Hp[slot].copy_(g.H.reshape(-1))
+    hp = _native.WaamCopyPlane(tape.at("Hp", slot), g.H.data_ptr(), 4 * g.n_cells)
+    _call("waam_copy_planes", ctypes.byref(hp), 1, st)
     _native.call("waam_step_main", ctypes.byref(f), ctypes.byref(p), ws.data_ptr(), ws.numel(),
                  st)
     g._forces_dirty = False

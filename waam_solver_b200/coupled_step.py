@@ -469,7 +469,7 @@ def flush_stream(g):
     g._collide_pending = False
     g._lag_pending = False      # a held stream is pending only with a collision (_pending_params)
     kernels.PENDING_GRIDS.discard(g)
-    st = torch.cuda.current_stream().cuda_stream
+    st = _native.stream_handle()
     if collide:
         p = g._pending_params
         _native.call("waam_step_finish", ctypes.byref(_fields_cached(g)), ctypes.byref(p),
@@ -501,7 +501,7 @@ def _run_graph(twin, g, f, p, ws, key):
         side = torch.cuda.Stream()
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.graph(graph, stream=side):
-            st = torch.cuda.current_stream().cuda_stream
+            st = _native.stream_handle()
             _native.call("waam_step_pre", ctypes.byref(f), ctypes.byref(p), ws.data_ptr(),
                          ws.numel(), st)
             _native.call("waam_step_main", ctypes.byref(f), ctypes.byref(p), ws.data_ptr(),
@@ -618,7 +618,7 @@ def coupled_step_fused(twin, torch_x_m, torch_y_m, is_welding, torch_z_m=None):
                (dx_, dy_, dz_) if twin.enable_bead_freeze else None)
         done = _run_graph(twin, g, f, p, ws, key)
     if not done:
-        stream = torch.cuda.current_stream().cuda_stream
+        stream = _native.stream_handle()
         _native.call("waam_step_pre", ctypes.byref(f), ctypes.byref(p), ws.data_ptr(),
                      ws.numel(), stream)
         if due:

@@ -26,11 +26,18 @@ _W = [1.0 / 3.0] + [1.0 / 18.0] * 6 + [1.0 / 36.0] * 12
 
 def _flags_ok(**kw):
     for k, v in kw.items():
-        if int(v) != FLAG_VALUES[k]:
+        if v != FLAG_VALUES[k] and int(v) != FLAG_VALUES[k]:
             raise WaamError("%s=%s differs from the built-in value %d" % (k, v, FLAG_VALUES[k]))
 
 
+_F32, _I32, _Tensor = torch.float32, torch.int32, torch.Tensor
+
+
 def _f(t, n=None):
+    # one test for the ordinary argument; the messages only for a wrong one
+    if (isinstance(t, _Tensor) and t.dtype is _F32 and t.is_cuda and t.is_contiguous() and
+            (n is None or t.numel() == n)):
+        return t.data_ptr()
     if not isinstance(t, torch.Tensor) or not t.is_cuda:
         raise WaamError("expected a CUDA tensor, got %r" % type(t))
     if t.dtype != torch.float32 or not t.is_contiguous():
@@ -57,6 +64,9 @@ def _pop(t, n=None):
 
 
 def _i(t, n=None):
+    if (isinstance(t, _Tensor) and t.dtype is _I32 and t.is_cuda and t.is_contiguous() and
+            (n is None or t.numel() == n)):
+        return t.data_ptr()
     if not isinstance(t, torch.Tensor) or not t.is_cuda:
         raise WaamError("expected a CUDA tensor, got %r" % type(t))
     if t.dtype != torch.int32 or not t.is_contiguous():
@@ -72,8 +82,7 @@ def _dims(t):
     return tuple(t.shape)
 
 
-def _stream():
-    return torch.cuda.current_stream().cuda_stream
+_stream = _native.stream_handle
 
 
 _WORKSPACES = {}
@@ -123,16 +132,22 @@ IN_FUSED_STEP = [False]
 def state_changed():
     """Record a change of flags / phi / f_l / H / T made outside the fused step,
     after running the work a pipelined step left pending."""
-    if not IN_FUSED_STEP[0]:
+    if not IN_FUSED_STEP[0] and PENDING_GRIDS:
         for g in list(PENDING_GRIDS):
             g.flush_stream()
     STATE_EPOCH[0] += 1
 
 
+_STATE_WRITERS = _TILE_STATE_WRITERS | _POPULATION_WRITERS
+
+
 def _call(name, *args):
-    if name in _TILE_STATE_WRITERS or name in _POPULATION_WRITERS:
+    if name in _STATE_WRITERS:
         state_changed()
-    return _native.call(name, *args)
+    rc = _native.function(name)(*args)
+    if rc != 0:
+        _native.check(name, rc)
+    return rc
 
 
 # ---------------------------------------------------------------- init ----
@@ -1038,15 +1053,21 @@ def extract_fl_yz_slice(f_l, out, i_slice, ny, nz):
     out.copy_(f_l[int(i_slice)].reshape(out.shape))
 
 
-def probe_sample(T, f_l, cells, row):
-    """T and f_l at cell indices ``cells`` (-1: outside) into ``row`` (device,
-    2 floats per probe), export/probes.py:90-107."""
+def probe_set(cells):
+    """WaamProbeSet of cell indices ``cells`` (-1: outside)."""
     if len(cells) > _native.MAX_PROBES:
         raise WaamError("at most %d probes" % _native.MAX_PROBES)
     ps = _native.WaamProbeSet()
     ps.n_probes = len(cells)
     for q, c in enumerate(cells):
         ps.cell[q] = int(c)
+    return ps
+
+
+def probe_sample(T, f_l, cells, row):
+    """T and f_l at cell indices ``cells`` (-1: outside) into ``row`` (device,
+    2 floats per probe), export/probes.py:90-107."""
+    ps = probe_set(cells)
     _call("waam_probe_sample", _f(T), _f(f_l), ctypes.byref(ps), _f(row), _stream())
 
 
