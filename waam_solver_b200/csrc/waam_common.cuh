@@ -89,11 +89,13 @@ struct Dims {
     int nx, ny, nz;
     __host__ __device__ int64_t n() const { return (int64_t)nx * ny * nz; }
     __host__ __device__ int idx(int i, int j, int k) const { return (i * ny + j) * nz + k; }
-    __device__ void ijk(int64_t c, int& i, int& j, int& k) const {
-        k = (int)(c % nz);
-        int64_t r = c / nz;
-        j = (int)(r % ny);
-        i = (int)(r / ny);
+    // 32-bit divisions (a cell index fits): 64-bit ones were most of the
+    // instructions of the operators' stencil kernels
+    __device__ __forceinline__ void ijk(int64_t c, int& i, int& j, int& k) const {
+        const unsigned u = (unsigned)c, r = u / (unsigned)nz;
+        k = (int)(u - r * (unsigned)nz);
+        i = (int)(r / (unsigned)ny);
+        j = (int)(r - (unsigned)i * (unsigned)ny);
     }
 };
 

@@ -481,6 +481,31 @@ __global__ void __launch_bounds__(256) k_arc_norm_tiles(Dims d, const int32_t* _
     // the surface query needs no launch of its own; block 0 publishes it
     __shared__ float s_arc_k;
     __shared__ float s_wd[kArcTableMax];
+    const int kt = (d.nz + kTileK - 1) / kTileK, jt = (d.ny + kTileJ - 1) / kTileJ;
+    const int tiles = kt * jt * d.nx;
+    // four tiles per pass: their flags and liquid fractions are all requested
+    // before any weight is computed (f_l of gas cells is read and ignored),
+    // the first pass's before the surface query
+    constexpr int kU = 4;
+    int fg[kU], ci[kU], cj[kU], ck[kU];
+    float fl[kU];
+    auto load = [&](int t0) {
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int t = t0 + u * gridDim.x;
+            const int a = t % kt, r = t / kt;
+            const int b = r % jt, i = r / jt;
+            const int k = a * kTileK + threadIdx.x, j = b * kTileJ + threadIdx.y;
+            const bool ok = t < tiles && k < d.nz && j < d.ny;
+            const int c = ok ? (i * d.ny + j) * d.nz + k : 0;
+            fg[u] = ok ? flags[c] : GAS;
+            fl[u] = ok ? f_l[c] : 0.0f;
+            ci[u] = i;
+            cj[u] = j;
+            ck[u] = k;
+        }
+    };
+    load(blockIdx.x);
     if (threadIdx.y == 0) {
         const float kf = surface_arc_k(d, phi, flags, scalars, nz_solid);
         if (threadIdx.x == 0) {
@@ -497,29 +522,8 @@ __global__ void __launch_bounds__(256) k_arc_norm_tiles(Dims d, const int32_t* _
         for (int k = threadIdx.y * kTileK + threadIdx.x; k < d.nz; k += kTileK * kTileJ)
             s_wd[k] = arc_weight(k, p.arc_k, 0.0f, p.pen, p.enable);
     __syncthreads();
-    const int kt = (d.nz + kTileK - 1) / kTileK, jt = (d.ny + kTileJ - 1) / kTileJ;
-    const int tiles = kt * jt * d.nx;
-    // four tiles per pass: their flags and liquid fractions are all requested
-    // before any weight is computed (f_l of gas cells is read and ignored)
-    constexpr int kU = 4;
     double part = 0.0;
-    for (int t0 = blockIdx.x; t0 < tiles; t0 += kU * gridDim.x) {
-        int fg[kU], ci[kU], cj[kU], ck[kU];
-        float fl[kU];
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            const int t = t0 + u * gridDim.x;
-            const int a = t % kt, r = t / kt;
-            const int b = r % jt, i = r / jt;
-            const int k = a * kTileK + threadIdx.x, j = b * kTileJ + threadIdx.y;
-            const bool ok = t < tiles && k < d.nz && j < d.ny;
-            const int c = ok ? (i * d.ny + j) * d.nz + k : 0;
-            fg[u] = ok ? flags[c] : GAS;
-            fl[u] = ok ? f_l[c] : 0.0f;
-            ci[u] = i;
-            cj[u] = j;
-            ck[u] = k;
-        }
+    for (int t0 = blockIdx.x; t0 < tiles;) {
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
             if (fg[u] == GAS) continue;
@@ -531,6 +535,8 @@ __global__ void __launch_bounds__(256) k_arc_norm_tiles(Dims d, const int32_t* _
             shape[(ci[u] * d.ny + cj[u]) * d.nz + ck[u]] = sh;
             part += (double)(sh * wd);
         }
+        t0 += kU * gridDim.x;
+        if (t0 < tiles) load(t0);
     }
     part = tile_block_sum(part);
     __shared__ bool last;
@@ -646,61 +652,109 @@ __global__ void __launch_bounds__(32 * kClassifyWarps)
     }
 }
 
+// Warp sums of eight values at once: lane l ends with the sum of value l >> 2
+// over the warp (its tree is that of a shuffle-down sum of that value alone).
+// 9 shuffles in place of 40.
+__device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
+#pragma unroll
+    for (int h = 4, o = 16; h >= 1; h >>= 1, o >>= 1) {
+        const bool hi = (lane & o) != 0;
+#pragma unroll
+        for (int u = 0; u < h; ++u) {
+            const double send = hi ? v[u] : v[u + h], keep = hi ? v[u + h] : v[u];
+            v[u] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    double t = v[0];
+    t += __shfl_xor_sync(0xffffffffu, t, 2);
+    t += __shfl_xor_sync(0xffffffffu, t, 1);
+    return t;
+}
+
 // The arc weight sum over the tiles of the work list (quiet tiles are all GAS
 // and weigh nothing).  Each listed tile's sum goes to its own slot of
 // tile_part (k_classify_tiles zeroes the quiet tiles' slots); the last block
 // adds all slots in tile order, so the total does not depend on the list's
 // order.  The surface query's arc k comes from k_classify_tiles.  A block
-// takes kArcBatch listed tiles at a time: their loads are all issued first and
-// their block sums share one barrier.  Otherwise as k_arc_norm_tiles.
+// takes kArcBatch listed tiles at a time, gridDim.x apart (so that a short
+// list still reaches every block): their loads are all issued first -- the
+// first batch's before the tables are built -- and their block sums share one
+// barrier.  Latency decides: the last block's sum of the slots, a chain of
+// four loads at a time, was half of the kernel on 512x256x160 (81,920 slots).
 constexpr int kArcBatch = 8;
-__global__ void __launch_bounds__(256) k_arc_norm_list(Dims d, const int32_t* __restrict__ flags,
+__global__ void __launch_bounds__(256, 4) k_arc_norm_list(Dims d, const int32_t* __restrict__ flags,
                                                        const float* __restrict__ f_l,
                                                        ArcParams p, float* scalars,
                                                        float arc_k_offset, float Qe_dt, float dx3,
                                                        Workspace ws, float* __restrict__ shape,
                                                        const int32_t* __restrict__ list,
                                                        double* __restrict__ tile_part, int tiles) {
+    constexpr int kU = kArcBatch, kWarps = (kTileK * kTileJ) / 32;
+    static_assert(kU == 8, "warp_sum8 takes a batch");
     __shared__ float s_wd[kArcTableMax];
-    p.arc_k = scalars[kScalarArcK] + arc_k_offset;
-    p.arc_i = scalars[kScalarArcI];
-    p.arc_j = scalars[kScalarArcJ];
-    const bool table = d.nz <= kArcTableMax;
-    if (table)
-        for (int k = threadIdx.y * kTileK + threadIdx.x; k < d.nz; k += kTileK * kTileJ)
-            s_wd[k] = arc_weight(k, p.arc_k, 0.0f, p.pen, p.enable);
-    // The spatial factor's exponent is a sum of an i, a j and a k term
-    // (Gaussian: di^2 + dj^2 + dk^2 / 4; Goldak: xt^2 / a^2 + dj^2 / b^2 +
-    // dk^2 / c^2, waam_common.cuh arc_cell_shape); each term is tabulated once
-    // per block with the per-cell expression and added in the same order, so
-    // a cell costs one exponential and no division.
     __shared__ float s_axis[kArcAxisMax];
+    __shared__ double s_part[kU][kWarps];
+    __shared__ bool last;
+    const int tid = threadIdx.y * kTileK + threadIdx.x, lane = threadIdx.x;
+    const int cnt = imin(list[0], tiles);
+    const bool table = d.nz <= kArcTableMax;
     const bool axes = d.nx + d.ny + d.nz <= kArcAxisMax;
-    if (axes) {
-        const float eps = 1e-6f;
-        for (int t = threadIdx.y * kTileK + threadIdx.x; t < d.nx + d.ny + d.nz;
-             t += kTileK * kTileJ) {
-            float v;
-            if (t < d.nx) {
-                const float di = (float)t - p.arc_i;
-                if (p.kind == 0) {
-                    v = di * di;
-                } else {
-                    const float xt = di * p.sign;
-                    const float a = xt >= 0.0f ? p.a_f : p.a_r;
-                    v = (xt * xt) / (a * a + eps);
-                }
-            } else if (t < d.nx + d.ny) {
-                const float dj = (float)(t - d.nx) - p.arc_j;
-                v = p.kind == 0 ? dj * dj : (dj * dj) / (p.b * p.b + eps);
-            } else {
-                const float dk = (float)(t - d.nx - d.ny) - p.arc_k;
-                v = p.kind == 0 ? dk * dk * 0.25f : (dk * dk) / (p.c * p.c + eps);
-            }
-            s_axis[t] = v;
+    int ent[kU], fg[kU], ck[kU];
+    float fl[kU];
+    auto load = [&](int e0) {
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int e = e0 + u * (int)gridDim.x;
+            ent[u] = e < cnt ? list[1 + e] : -1;
         }
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            int i = 0, j = 0, k = 0, c = 0;
+            const bool ok = ent[u] >= 0 && list_tile_cell(d, ent[u], i, j, k, c);
+            fg[u] = ok ? flags[c] : GAS;
+            fl[u] = ok ? f_l[c] : 0.0f;
+            ck[u] = k;
+        }
+    };
+    int e0 = blockIdx.x;
+    if (e0 < cnt) {
+        load(e0);
+        p.arc_k = scalars[kScalarArcK] + arc_k_offset;
+        p.arc_i = scalars[kScalarArcI];
+        p.arc_j = scalars[kScalarArcJ];
+        if (table)
+            for (int k = tid; k < d.nz; k += kTileK * kTileJ)
+                s_wd[k] = arc_weight(k, p.arc_k, 0.0f, p.pen, p.enable);
+        // The spatial factor's exponent is a sum of an i, a j and a k term
+        // (Gaussian: di^2 + dj^2 + dk^2 / 4; Goldak: xt^2 / a^2 + dj^2 / b^2 +
+        // dk^2 / c^2, waam_common.cuh arc_cell_shape); each term is tabulated
+        // once per block with the per-cell expression and added in the same
+        // order, so a cell costs one exponential and no division.
+        if (axes) {
+            const float eps = 1e-6f;
+            for (int t = tid; t < d.nx + d.ny + d.nz; t += kTileK * kTileJ) {
+                float v;
+                if (t < d.nx) {
+                    const float di = (float)t - p.arc_i;
+                    if (p.kind == 0) {
+                        v = di * di;
+                    } else {
+                        const float xt = di * p.sign;
+                        const float a = xt >= 0.0f ? p.a_f : p.a_r;
+                        v = (xt * xt) / (a * a + eps);
+                    }
+                } else if (t < d.nx + d.ny) {
+                    const float dj = (float)(t - d.nx) - p.arc_j;
+                    v = p.kind == 0 ? dj * dj : (dj * dj) / (p.b * p.b + eps);
+                } else {
+                    const float dk = (float)(t - d.nx - d.ny) - p.arc_k;
+                    v = p.kind == 0 ? dk * dk * 0.25f : (dk * dk) / (p.c * p.c + eps);
+                }
+                s_axis[t] = v;
+            }
+        }
+        __syncthreads();
     }
-    __syncthreads();
     auto shape_of = [&](int i, int j, int k) -> float {
         if (!axes) return arc_cell_shape(p, i, j, k);
         const float sum = (s_axis[i] + s_axis[d.nx + j]) + s_axis[d.nx + d.ny + k];
@@ -708,42 +762,26 @@ __global__ void __launch_bounds__(256) k_arc_norm_list(Dims d, const int32_t* __
         const float xt = ((float)i - p.arc_i) * p.sign;
         return (xt >= 0.0f ? p.ff : p.fr) * waam_expf(-3.0f * sum);
     };
-    const int tid = threadIdx.y * kTileK + threadIdx.x;
-    const int cnt = imin(list[0], tiles);
-    constexpr int kU = kArcBatch, kWarps = (kTileK * kTileJ) / 32;
-    __shared__ double s_part[kU][kWarps];
-    for (int e0 = blockIdx.x * kU; e0 < cnt; e0 += kU * gridDim.x) {
-        int ent[kU];
-#pragma unroll
-        for (int u = 0; u < kU; ++u) ent[u] = e0 + u < cnt ? list[1 + e0 + u] : -1;
-        int fg[kU], ci[kU], cj[kU], ck[kU];
-        float fl[kU];
+    while (e0 < cnt) {
+        double v[kU];
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
-            int i = 0, j = 0, k = 0, c = 0;
-            const bool ok = ent[u] >= 0 && list_tile_cell(d, ent[u], i, j, k, c);
-            fg[u] = ok ? flags[c] : GAS;
-            fl[u] = ok ? f_l[c] : 0.0f;
-            ci[u] = i;
-            cj[u] = j;
-            ck[u] = k;
-        }
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            double v = 0.0;
+            v[u] = 0.0;
             if (fg[u] != GAS) {
                 const float wd = !table ? arc_weight(ck[u], p.arc_k, fl[u], p.pen, p.enable)
                                         : (fl[u] > 0.55f ? 1.0f : s_wd[ck[u]]);
                 if (!(wd < 1e-6f)) {
-                    const float sh = shape_of(ci[u], cj[u], ck[u]);
-                    shape[(ci[u] * d.ny + cj[u]) * d.nz + ck[u]] = sh;
-                    v = (double)(sh * wd);
+                    int i, j, k, c;
+                    list_tile_cell(d, ent[u], i, j, k, c);
+                    const float sh = shape_of(i, j, k);
+                    shape[c] = sh;
+                    v[u] = (double)(sh * wd);
                 }
             }
-            // the block sum of tile_block_sum: warp tree, then the warps in order
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-            if ((tid & 31) == 0) s_part[u][tid >> 5] = v;
         }
+        // the block sums of tile_block_sum: warp tree, then the warps in order
+        const double t = warp_sum8(v, lane);
+        if ((lane & 3) == 0) s_part[lane >> 2][tid >> 5] = t;
         __syncthreads();
         int mine = -1;   // thread u < kU writes tile u's slot
 #pragma unroll
@@ -754,10 +792,13 @@ __global__ void __launch_bounds__(256) k_arc_norm_list(Dims d, const int32_t* __
             for (int w = 0; w < kWarps; ++w) sum += s_part[tid][w];
             tile_part[tile_index(d, mine)] = sum;
         }
+        e0 += kU * (int)gridDim.x;
+        if (e0 < cnt) load(e0);
         __syncthreads();
     }
-    __shared__ bool last;
     if (tid == 0) {
+        // thread 0 wrote its slot itself; the others' are ordered before this
+        // by the barrier above
         __threadfence();
         const unsigned prev = atomicAdd(ws.counter, 1u);
         last = prev == gridDim.x - 1;
@@ -766,10 +807,20 @@ __global__ void __launch_bounds__(256) k_arc_norm_list(Dims d, const int32_t* __
     if (!last) return;
     __threadfence();
     // the slots come from other blocks (fenced before their arrival count):
-    // read them from L2 (__ldcg), independent loads that can all be in flight;
-    // a quiet tile's slot is 0 and adds nothing
+    // read them from L2 (__ldcg), sixteen independent loads at a time; a quiet
+    // tile's slot is 0 and adds nothing
     double acc = 0.0;
-    for (int t = tid; t < tiles; t += kTileK * kTileJ) acc += __ldcg(tile_part + t);
+    constexpr int kL = 16, kT = kTileK * kTileJ;
+    for (int t0 = tid; t0 < tiles; t0 += kL * kT) {
+        double x[kL];
+#pragma unroll
+        for (int u = 0; u < kL; ++u) {
+            const int t = t0 + u * kT;
+            x[u] = t < tiles ? __ldcg(tile_part + t) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < kL; ++u) acc += x[u];
+    }
     const double tot = tile_block_sum(acc);
     if (tid == 0) {
         *ws.counter = 0u;
@@ -784,14 +835,10 @@ __global__ void __launch_bounds__(256) k_arc_norm_list(Dims d, const int32_t* __
 // Pass 2 for one cell: H += epw * weight (non-gas cells), then the enthalpy
 // ceiling (solvers/coupled_step.py:107-108); wd_dry is the depth weight of
 // the cell's k for a cell that is not liquid.
-__device__ __forceinline__ void inject_cell(float* __restrict__ H, const int32_t* __restrict__ flags,
-                                            const float* __restrict__ f_l, float epw, int cap,
-                                            const PhaseParams& ph, const float* __restrict__ cp_f,
-                                            const VarPhase& vp, const float* __restrict__ shape,
-                                            float wd_dry, int c) {
-    const int flag = flags[c];
-    const float fl = f_l[c];           // requested with the flag (ignored for gas cells)
-    float h = cap ? H[c] : 0.0f;
+__device__ __forceinline__ void inject_value(float* __restrict__ H, int flag, float fl, float h,
+                                             float sh, float epw, int cap, const PhaseParams& ph,
+                                             const float* __restrict__ cp_f, const VarPhase& vp,
+                                             float wd_dry, int c) {
     if (flag == GAS) return;
     // arc_cell_heat (waam_common.cuh) with the spatial factor the weight-sum
     // pass left in `shape` and the depth weight from the table
@@ -800,7 +847,7 @@ __device__ __forceinline__ void inject_cell(float* __restrict__ H, const int32_t
     if (epw > 0.0f) {
         const float wd = fl > 0.55f ? 1.0f : wd_dry;
         if (!(wd < 1e-6f)) {
-            dh = epw * shape[c] * wd;
+            dh = epw * sh * wd;
             hit = true;
         }
     }
@@ -811,6 +858,17 @@ __device__ __forceinline__ void inject_cell(float* __restrict__ H, const int32_t
     // (kernels.py:1988-2010)
     if (cap) h = cp_f ? cap_h_var(vp, cp_f[c], h) : cap_h(ph, h);
     H[c] = h;
+}
+
+__device__ __forceinline__ void inject_cell(float* __restrict__ H, const int32_t* __restrict__ flags,
+                                            const float* __restrict__ f_l, float epw, int cap,
+                                            const PhaseParams& ph, const float* __restrict__ cp_f,
+                                            const VarPhase& vp, const float* __restrict__ shape,
+                                            float wd_dry, int c) {
+    const int flag = flags[c];
+    const float fl = f_l[c];           // requested with the flag (ignored for gas cells)
+    const float h = cap ? H[c] : 0.0f;
+    inject_value(H, flag, fl, h, shape[c], epw, cap, ph, cp_f, vp, wd_dry, c);
 }
 
 __global__ void __launch_bounds__(256) k_arc_inject_tiles(Dims d, float* __restrict__ H,
@@ -856,12 +914,36 @@ __global__ void __launch_bounds__(256) k_arc_inject_list(Dims d, float* __restri
             s_wd[k] = arc_weight(k, p.arc_k, 0.0f, p.pen, p.enable);
     __syncthreads();
     const float epw = scalars[kScalarEpw];
-    for_list_tiles(list, imin(list[0], tiles), [&](int ent) {
-        int i, j, k, c;
-        if (!list_tile_cell(d, ent, i, j, k, c)) return;
-        const float wd = table ? s_wd[k] : arc_weight(k, p.arc_k, 0.0f, p.pen, p.enable);
-        inject_cell(H, flags, f_l, epw, cap, ph, cp_f, vp, shape, wd, c);
-    });
+    // four tiles at a time, every load of theirs (the shape factor of cells
+    // that have none included) before any store
+    constexpr int kU = 4;
+    const int cnt = imin(list[0], tiles);
+    for (int e0 = blockIdx.x; e0 < cnt; e0 += kU * (int)gridDim.x) {
+        int cell[kU], fg[kU], kk[kU];
+        float fl[kU], h[kU], sh[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int e = e0 + u * (int)gridDim.x;
+            cell[u] = e < cnt ? list[1 + e] : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            int i, j, k = 0, c = 0;
+            const bool ok = cell[u] >= 0 && list_tile_cell(d, cell[u], i, j, k, c);
+            cell[u] = c;
+            kk[u] = k;
+            fg[u] = ok ? flags[c] : GAS;
+            fl[u] = ok ? f_l[c] : 0.0f;
+            h[u] = ok && cap ? H[c] : 0.0f;
+            sh[u] = ok ? shape[c] : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            if (fg[u] == GAS) continue;
+            const float wd = table ? s_wd[kk[u]] : arc_weight(kk[u], p.arc_k, 0.0f, p.pen, p.enable);
+            inject_value(H, fg[u], fl[u], h[u], sh[u], epw, cap, ph, cp_f, vp, wd, cell[u]);
+        }
+    }
 }
 
 struct ThermalArgs {
