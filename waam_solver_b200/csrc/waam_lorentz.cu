@@ -216,7 +216,8 @@ inline unsigned row_blocks(const RowGrid& g) {
 template <int V>
 __device__ __forceinline__ bool row_cells(const RowGrid& g, int& i, int& j, int& k, int& c) {
     constexpr int kLanes = 32 / V;   // lanes per column
-    const unsigned w = (blockIdx.x * kThreads + threadIdx.x) >> 5;
+    // counted in warps: the threads of more than 2^27 of them pass 32 bits
+    const unsigned w = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     const unsigned cg = g.by_kt.div(w);
     const int col = (int)cg * V + lane / kLanes;
