@@ -62,3 +62,24 @@ def test_arc_source_of_the_last_columns():
     # the scale divides by a double sum taken in another order: one unit of
     # float32 in the sum, one in the quotient
     assert bool(((out[0] - out[1]).abs() <= 2.0 ** -22 * out[1].abs()).all())
+
+
+def test_arc_source_on_the_most_columns():
+    """65534 x 32769 columns of one cell (2^31 - 2): the weight sum's stride past
+    the last column does not fit 31 bits."""
+    import torch
+    from waam_solver_b200 import _native
+    nx, ny = 65534, 32769
+    out = []
+    for m in (nx, 64):
+        src = torch.empty((m, ny, 1), dtype=torch.float32, device="cuda")
+        src[-ROWS:].fill_(float("nan"))
+        ws = torch.zeros(int(_native.lib().waam_workspace_bytes(m * ny)), dtype=torch.uint8,
+                         device="cuda")
+        _native.call("waam_elec_arc_source", src.data_ptr(), m, ny, 1, m - 5.75, 4000.25, 0.5, 3.0,
+                     140.0, 2e-4, ws.data_ptr(), ws.numel(), _native.stream_handle())
+        out.append(src[-ROWS:].clone())
+        del src, ws
+        torch.cuda.empty_cache()
+    assert bool((out[0] > 0.0).any())
+    assert bool(((out[0] - out[1]).abs() <= 2.0 ** -22 * out[1].abs()).all())

@@ -251,9 +251,11 @@ __global__ void __launch_bounds__(kTileK* kTileJ)
     source_slab(arc_k, sigma_cells, d.nz, k_min, k_max);
     double part = 0.0;
     const int ks = imax(k_min, 0), ke = imin(k_max, d.nz - 1);
-    const int ncol = d.nx * d.ny, lane = threadIdx.x;
-    for (int col = blockIdx.x * kTileJ + threadIdx.y; col < ncol; col += gridDim.x * kTileJ) {
-        const int i = col / d.ny, j = col - i * d.ny;
+    const int lane = threadIdx.x;
+    // unsigned: one stride past the last of nearly 2^31 columns is still above it
+    const unsigned ncol = (unsigned)d.nx * (unsigned)d.ny;
+    for (unsigned col = blockIdx.x * kTileJ + threadIdx.y; col < ncol; col += gridDim.x * kTileJ) {
+        const int i = (int)(col / (unsigned)d.ny), j = (int)col - i * d.ny;
         const float di = (float)i - arc_i, dj = (float)j - arc_j;
         if (-(di * di + dj * dj) * inv2s2 < -104.0f) continue;
         for (int k = ks + lane; k <= ke; k += kTileK) {
