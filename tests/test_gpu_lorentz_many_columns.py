@@ -1,7 +1,7 @@
-"""The Lorentz field kernels on grids of more than 2^27 columns, where one warp
-per column is more than 2^32 threads: the last columns against the same columns
-of a small grid (the arc shifted by a whole number of cells, so that every
-distance is the same float)."""
+"""The Lorentz field kernels on grids of more than 2^27 columns or levels, where
+one warp for each is more than 2^32 threads: the last columns against the same
+columns of a small grid (the arc shifted by a whole number of cells, so that
+every distance is the same float), the levels against their own sums."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -83,3 +83,13 @@ def test_arc_source_on_the_most_columns():
         torch.cuda.empty_cache()
     assert bool((out[0] > 0.0).any())
     assert bool(((out[0] - out[1]).abs() <= 2.0 ** -22 * out[1].abs()).all())
+
+
+def test_bin_prefix_of_the_last_levels():
+    import torch
+    from waam_solver_b200 import kernels as K
+    nz = 2 ** 27 + 100
+    bins = torch.rand((nz, 2), device="cuda", generator=torch.Generator("cuda").manual_seed(9))
+    want = torch.stack((bins[:, 0], bins[:, 0] + bins[:, 1]), dim=1)
+    K.elec_prefix_bins(bins, 2, nz)
+    assert torch.equal(bins, want)

@@ -844,7 +844,8 @@ __global__ void k_elec_bin_store(const double* acc, float* bins, int64_t m) {
 // bins loaded 32 at a time and added one after another through shuffles (the
 // float order of the reference).
 __global__ void __launch_bounds__(256) k_elec_prefix(float* bins, int n_bins, int nz) {
-    const int k = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    const int k = (int)(blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5));
+    const int lane = threadIdx.x & 31;
     if (k >= nz) return;
     float a = 0.0f;
     for (int b0 = 0; b0 < n_bins; b0 += 32) {
