@@ -50,11 +50,29 @@ def _ptr(t):
 _stream = _native.stream_handle
 
 
+def _on_current_device(t):
+    return t.is_cuda and t.device.index == torch.cuda.current_device()
+
+
+def _raw_copy(dst, src):
+    """Whether dst.copy_(src) is a copy of src's bytes that the kernel can make."""
+    return (dst.shape == src.shape and dst.dtype == src.dtype and dst.device == src.device and
+            dst.is_contiguous() and src.is_contiguous() and
+            src.numel() * src.element_size() % 4 == 0 and _on_current_device(src))
+
+
 def _copy_planes(pairs):
-    """dst <- src for every (dst, src) pair of contiguous tensors, in one launch
-    (per 32 of them)."""
-    for s0 in range(0, len(pairs), _native.MAX_COPY_PLANES):
-        part = pairs[s0:s0 + _native.MAX_COPY_PLANES]
+    """dst.copy_(src) for every (dst, src) pair, the plain copies in one launch
+    (per 32 of them); the others convert, or raise, as copy_ does, before any
+    plain one is made."""
+    raw = []
+    for dst, src in pairs:
+        if _raw_copy(dst, src):
+            raw.append((dst, src))
+        else:
+            dst.copy_(src)
+    for s0 in range(0, len(raw), _native.MAX_COPY_PLANES):
+        part = raw[s0:s0 + _native.MAX_COPY_PLANES]
         table = (_native.WaamCopyPlane * len(part))()
         for row, (dst, src) in zip(table, part):
             row.dst, row.src = dst.data_ptr(), src.data_ptr()
@@ -122,6 +140,26 @@ class _Tape:
         # the double buffers: they hold for the grid's fields while this tape lives
         self._fields, self._tables = {}, {}
 
+        for name, t in self._recorded(g) + [("Hp", g.H), ("H", g.H_next), ("T", g.T_next)]:
+            self._check(name, t)
+
+    @staticmethod
+    def _recorded(g):
+        """(record, field) of the state after a step; u holds three fields."""
+        return [("H", g.H), ("T", g.T), ("fl", g.f_l), ("phi", g.phi), ("flags", g.flags),
+                ("u", g.ux), ("u", g.uy), ("u", g.uz), ("scal", g.step_scalars)]
+
+    def _check(self, name, t):
+        """The records are copied by address: a field of another size, type or
+        order than its slot raises."""
+        rec = getattr(self, name)
+        size = self._at[name][1] // (3 if name == "u" else 1)
+        if (t.numel() * t.element_size() != size or t.dtype != rec.dtype or
+                t.device != rec.device or not t.is_contiguous()):
+            raise WaamError("adjoint tape: a %s %s field does not fit record '%s' (%d bytes)"
+                            % (tuple(t.shape), t.dtype, name, size))
+        return size
+
     def at(self, name, slot):
         """Device address of a record (an index into the tensor costs more than
         the launch it is for)."""
@@ -144,11 +182,10 @@ class _Tape:
         """The state after a step into its slot."""
         entry = self._tables.get(g._cur)
         if entry is None:
-            src = (("H", g.H), ("T", g.T), ("fl", g.f_l), ("phi", g.phi), ("flags", g.flags),
-                   ("u", g.ux), ("u", g.uy), ("u", g.uz), ("scal", g.step_scalars))
+            src = self._recorded(g)
             rows = (_native.WaamCopyPlane * len(src))()
-            for row, (_, t) in zip(rows, src):
-                row.src, row.bytes = t.data_ptr(), t.numel() * t.element_size()
+            for row, (name, t) in zip(rows, src):
+                row.src, row.bytes = t.data_ptr(), self._check(name, t)
             entry = self._tables[g._cur] = rows, [name for name, _ in src]
         rows, names = entry
         n3 = self._at["u"][1] // 3
@@ -258,7 +295,10 @@ class AdjointProblem:
         self.hist = torch.zeros((self.N, max(2 * P, 2)), dtype=torch.float32, device=g.device)
         self.scal = torch.zeros((self.N, 16), dtype=torch.float32, device=g.device)
         self.checkpoints = {}
-        row = _native.WaamCopyPlane(bytes=64)
+        if not _raw_copy(self.scal[0], g.step_scalars):
+            raise WaamError("the step scalars are not %d floats" % self.scal.shape[1])
+        scal_row = 4 * self.scal.shape[1]
+        row = _native.WaamCopyPlane(bytes=scal_row)
         scal_at, hist_at = self.scal.data_ptr(), self.hist.data_ptr()
         hist_row = 4 * self.hist.shape[1]
         probes = kernels.probe_set(self.cell_list)
@@ -266,7 +306,7 @@ class AdjointProblem:
             if n % self.K == 0:
                 self.checkpoints[n] = _Checkpoint(tw)
             tw.step(x, y, True)
-            row.dst, row.src = scal_at + 64 * n, g.step_scalars.data_ptr()
+            row.dst, row.src = scal_at + scal_row * n, g.step_scalars.data_ptr()
             _call("waam_copy_planes", ctypes.byref(row), 1, _stream())
             if P:
                 _call("waam_probe_sample", g.T.data_ptr(), g.f_l.data_ptr(), ctypes.byref(probes),
