@@ -676,12 +676,18 @@ __device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
 // tile_part (k_classify_tiles zeroes the quiet tiles' slots); the last block
 // adds all slots in tile order, so the total does not depend on the list's
 // order.  The surface query's arc k comes from k_classify_tiles.  A block
-// takes kArcBatch listed tiles at a time, gridDim.x apart (so that a short
-// list still reaches every block): their loads are all issued first -- the
-// first batch's before the tables are built -- and their block sums share one
-// barrier.  Latency decides: the last block's sum of the slots, a chain of
+// takes kArcBatch listed tiles at a time: their loads are all issued first --
+// the first batch's before the tables are built -- and their block sums share
+// one barrier.  Latency decides: the last block's sum of the slots, a chain of
 // four loads at a time, was half of the kernel on 512x256x160 (81,920 slots).
+// A short list goes to as many blocks as get kArcShare tiles each, one per SM
+// at least: further blocks wait for registers of the collision and the stream
+// beside them, and the sum ends with the last.  A step of 116x58x43 (about 950
+// tiles), 100x50x50 (700) and 128x64x48 (1050): 64.6, 52.7 and 69.6 us; on all
+// 592 blocks 66.0, 56.2 and 69.7; with five tiles each 64.0, 53.2 and 70.6.
 constexpr int kArcBatch = 8;
+constexpr int kArcShare = 3;
+constexpr int kArcMinBlocks = 148;
 __global__ void __launch_bounds__(256, 4) k_arc_norm_list(Dims d, const int32_t* __restrict__ flags,
                                                        const float* __restrict__ f_l,
                                                        ArcParams p, float* scalars,
@@ -699,12 +705,13 @@ __global__ void __launch_bounds__(256, 4) k_arc_norm_list(Dims d, const int32_t*
     const int cnt = imin(list[0], tiles);
     const bool table = d.nz <= kArcTableMax;
     const bool axes = d.nx + d.ny + d.nz <= kArcAxisMax;
+    const int busy = imin((int)gridDim.x, imax(kArcMinBlocks, (cnt + kArcShare - 1) / kArcShare));
     int ent[kU], fg[kU], ck[kU];
     float fl[kU];
     auto load = [&](int e0) {
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
-            const int e = e0 + u * (int)gridDim.x;
+            const int e = e0 + u * busy;
             ent[u] = e < cnt ? list[1 + e] : -1;
         }
 #pragma unroll
@@ -716,7 +723,7 @@ __global__ void __launch_bounds__(256, 4) k_arc_norm_list(Dims d, const int32_t*
             ck[u] = k;
         }
     };
-    int e0 = blockIdx.x;
+    int e0 = (int)blockIdx.x < busy ? (int)blockIdx.x : cnt;
     if (e0 < cnt) {
         load(e0);
         p.arc_k = scalars[kScalarArcK] + arc_k_offset;
@@ -792,7 +799,7 @@ __global__ void __launch_bounds__(256, 4) k_arc_norm_list(Dims d, const int32_t*
             for (int w = 0; w < kWarps; ++w) sum += s_part[tid][w];
             tile_part[tile_index(d, mine)] = sum;
         }
-        e0 += kU * (int)gridDim.x;
+        e0 += kU * busy;
         if (e0 < cnt) load(e0);
         __syncthreads();
     }
