@@ -72,8 +72,9 @@ def test_collide_srt_sums(backends, n, odd):
 @pytest.mark.parametrize("shape", [(1, 1, 1), (2, 1, 3), (3, 9, 31), (4, 8, 32), (5, 7, 65),
                                    (3, 2, 97)])
 def test_step_stream_at_row_ends(backends, storage, shape):
-    """The fused step's stream (which mends the bounced cells after its stores),
-    float32 and 2-byte elements, against the oracle's on the same values."""
+    """The fused step's stream in order, float32 and 2-byte elements, against the
+    oracle's on the same values (beside the next step's stages it mends the
+    bounced cells after its stores: test_gpu_lagged_stream.py)."""
     import ctypes
     import torch
     from waam_solver_b200 import _native

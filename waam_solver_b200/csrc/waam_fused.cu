@@ -275,14 +275,18 @@ __device__ __noinline__ void bounce_cell(const StreamGrid& g, const StreamPtrs<T
 __device__ __forceinline__ bool is_active(int flag) { return flag == FLUID || flag == IFACE; }
 
 // T is the stored element: streaming moves stored values unchanged, whatever
-// the population storage.  Two forms, for what their grids hold:
-// VOTE, the operator: any number of fluid cells; each warp votes on the SOLID
-// cells around it.  192x96x66 all fluid: 44.8 us against 64 with a flag load
-// per population (and 32-cell rows, a third of whose lanes nz = 66 left idle).
-// Else, the fused step: few cells bounce (the melt surface), so they are
-// mended after the stores and the kernel keeps the registers of a plain copy:
-// it runs beside the step's other kernels, and what a 256x128x96 step waits
-// for is its end (0.2149 ms per step; 0.2175 with the votes' 48 registers).
+// the population storage.  Two forms, for what runs beside them:
+// VOTE, alone on its stream (the operator, and a step's stream in order): each
+// warp votes on the SOLID cells around it, the flag loads beside the pulls.
+// 192x96x66 all fluid: 44.8 us against 64 with a flag load per population (and
+// 32-cell rows, a third of whose lanes nz = 66 left idle).  With the other
+// form, whose mending is a tail that nothing hides, steps with the remelt tail
+// take 3 % longer on 64x32x32 and 80x48x32, 1 % on 256x128x96 (and 0.5 % less
+// there with 2-byte elements).
+// Else, beside the next step's stages: few cells bounce (the melt surface), so
+// they are mended after the stores and the kernel keeps the registers of a
+// plain copy.  What a 256x128x96 step waits for is its end: with the votes'
+// 48 registers it takes 1.2 % longer.
 // next_flags (null: none): the flags of the step after the streamed one.
 // Cells active there (FLUID / IFACE) are left alone: that step's collision
 // writes all 19 populations of each of them into the buffer the stream
@@ -409,10 +413,20 @@ int launch_stream(Dims d, const float* f_src, float* f_dst, const int32_t* flags
     return check_launch("k_stream");
 }
 
-// The fused step's stream: 4-byte or 2-byte stored populations.
+// The fused step's stream in order (nothing runs beside it): 4-byte or 2-byte
+// stored populations.
 static int launch_stream_stored(Dims d, const void* f_src, void* f_dst, const int32_t* flags,
-                                int storage, cudaStream_t s,
-                                const int32_t* next_flags = nullptr) {
+                                int storage, cudaStream_t s) {
+    if (storage == kStoreF32)
+        launch_stream_t<float, true>(d, f_src, f_dst, flags, nullptr, s);
+    else
+        launch_stream_t<uint16_t, true>(d, f_src, f_dst, flags, nullptr, s);
+    return check_launch("k_stream");
+}
+
+// The pending or lagged stream, beside the next step's stages.
+static int launch_stream_beside(Dims d, const void* f_src, void* f_dst, const int32_t* flags,
+                                int storage, cudaStream_t s, const int32_t* next_flags = nullptr) {
     if (storage == kStoreF32)
         launch_stream_t<float, false>(d, f_src, f_dst, flags, next_flags, s);
     else
@@ -1888,7 +1902,7 @@ int waam_step_pre(const WaamFields* f, const WaamStepParams* p, void* workspace,
             // the buffer that collision reads into the one it writes, leaving
             // alone the cells that collision writes (active in the previous
             // step's flags); its own flags are the older copy
-            ea = launch_stream_stored(d, f->f_dst, f->f_src, f->flags_copy_rr, p->f_storage,
+            ea = launch_stream_beside(d, f->f_dst, f->f_src, f->flags_copy_rr, p->f_storage,
                                       aux->s3, f->flags_copy_r);
             if (ea) return ea;
         }
@@ -1898,7 +1912,7 @@ int waam_step_pre(const WaamFields* f, const WaamStepParams* p, void* workspace,
             // the flags it streams with: the previous step's copy if there is
             // one (then the column pass may rewrite the flags meanwhile)
             const int32_t* sf = f->flags_copy_r ? f->flags_copy_r : f->flags;
-            ea = launch_stream_stored(d, f->f_src, f->f_dst, sf, p->f_storage, aux->s3);
+            ea = launch_stream_beside(d, f->f_src, f->f_dst, sf, p->f_storage, aux->s3);
             if (ea) return ea;
         }
         // waam_step_main joins them before the column pass (without flag
@@ -1963,7 +1977,7 @@ int waam_step_finish(const WaamFields* f, const WaamStepParams* p, void* workspa
     int e = WAAM_OK;
     if (p->stream_lag) {
         // the stream held back by the previous step, then its collision
-        e = launch_stream_stored(d, f->f_dst, f->f_src, f->flags_copy_rr, p->f_storage, s,
+        e = launch_stream_beside(d, f->f_dst, f->f_src, f->flags_copy_rr, p->f_storage, s,
                                  f->flags_copy_r);
         if (e) return e;
     }
