@@ -1,7 +1,7 @@
-"""The reverse stream where its cells leave the common path: k faces (the
-clamped second destination, the bounce-back from a clamped source), j faces
-(the general loop) and the periodic x wrap, on grids down to one cell.  Exact
-transpose of the forward stream: <lam, S y> = <S^T lam, y>."""
+"""The reverse stream on the faces: y and z faces (up to three clamped
+destinations beside the common one, the bounce-back from a clamped source) and
+the periodic x wrap, on grids down to one cell.  Exact transpose of the forward
+stream: <lam, S y> = <S^T lam, y>."""
 import numpy as np
 import pytest
 

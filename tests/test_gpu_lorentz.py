@@ -143,13 +143,13 @@ def test_jacobi_chunk_matches_single_sweeps(n_sweeps):
     assert math.isclose(float(n1.item()), float(n2.item()), rel_tol=1e-6)
 
 
-@pytest.mark.parametrize("shape", [(40, 32, 28, 8), (70, 80, 40, 10)])
+@pytest.mark.parametrize("shape", [(40, 32, 28, 8), (70, 80, 40, 10), (115, 96, 96, 40)])
 def test_live_list_solve_matches_full_grid_sweeps(shape):
     """Three solves of 20 sweeps (chunks of 10) with the flags changing between
     them -- metal cells turning to gas and gas to metal -- on the live list and
     on full-grid sweeps: the potential in both buffers is equal bit for bit and
-    the L1 sums of every chunk agree.  The second grid has more than 1024 tile
-    blocks (two levels of the list's offset scan)."""
+    the L1 sums of every chunk agree.  The third grid has more than 1024 units
+    of 1024 cells (two levels of the list's offset scan)."""
     K = _k()
     dev = torch.device("cuda", 0)
     nx, ny, nz, nzs = shape
