@@ -123,7 +123,8 @@ _CTYPES = {
     "const WaamStepParams*": C.POINTER(WaamStepParams), "const char*": C.c_char_p,
     "void* const*": C.c_void_p, "const WaamMaterialTables*": C.POINTER(WaamMaterialTables),
     "WaamTelemetry*": C.c_void_p, "const WaamProbeSet*": C.POINTER(WaamProbeSet),
-    "const WaamShiftPlane*": C.c_void_p, "const WaamCopyPlane*": C.c_void_p, "const WaamExportChannel*": C.c_void_p,
+    "const WaamShiftPlane*": C.c_void_p, "const WaamCopyPlane*": C.c_void_p,
+    "const WaamExportChannel*": C.c_void_p,
     "double*": C.c_void_p, "uint8_t*": C.c_void_p, "const uint8_t*": C.c_void_p,
     "int64_t*": C.c_void_p, "unsigned long long*": C.c_void_p,
 }

@@ -28,8 +28,9 @@ namespace {
 constexpr int kAdjBlocks = 592;   // fixed, so the FP64 sums never depend on the GPU
 constexpr int kAdjThreads = 256;
 
-// Adds this launch's NR sums to out[NR]: per-block totals in fixed order,
-// the last block combines the partials in block order.
+// Adds this launch's NR sums to out[NR]: per-block totals in fixed order; in
+// the last block every thread adds a fixed strided share of the partials, then
+// the same tree, so the order never changes.
 template <int NR>
 __device__ void accumulate_sums(double (&v)[NR], Workspace ws, double* out) {
     __shared__ double sh[NR][kAdjThreads / 32];
@@ -54,10 +55,8 @@ __device__ void accumulate_sums(double (&v)[NR], Workspace ws, double* out) {
     __syncthreads();
     if (!last) return;
     __threadfence();
-    // every thread adds a fixed strided subset of each sum's partials, then the
-    // same tree as above: the order never changes (one thread adding 592
-    // partials one after another took most of the kernel's time; with it and
-    // the 32-bit cell decode, 128x64x48: inject 31.6 -> 18 us, mu 30.6 -> 11)
+    // (with one thread adding the 592 partials and 64-bit cell decodes,
+    // 128x64x48: inject 31.6 us against 18, mu 30.6 against 11)
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
         v[r] = 0.0;
@@ -77,13 +76,6 @@ __device__ void accumulate_sums(double (&v)[NR], Workspace ws, double* out) {
     if (threadIdx.x == 0) *ws.counter = 0u;
 }
 
-__device__ __forceinline__ void cell_ijk(const Dims& d, int64_t c, int& i, int& j, int& k) {
-    k = (int)(c % d.nz);
-    const int64_t r = c / d.nz;
-    j = (int)(r % d.ny);
-    i = (int)(r / d.ny);
-}
-
 // ---------------------------------------------------------------------------
 // Stream (kernels.py:2971-3010) transposed.  The pull writes X'[q][c] for
 // every non-solid c from Y'[q][src(c, q)], or, for a non-gas c whose source
@@ -94,12 +86,12 @@ __device__ __forceinline__ void cell_ijk(const Dims& d, int64_t c, int& i, int& 
 // ---------------------------------------------------------------------------
 // One source cell per thread, consecutive cells of the whole grid.  Population
 // q has the destination s + off(q) and, on a y / z face, up to three clamped
-// ones beside it (every row has face cells, so they take the common path, not
-// one of their own: a warp with a serial loop over its few face cells held the
-// kernel at 60 us on 128x64x48; 56 us with 32-cell rows, 41 us now).  The destinations' flags are turned into bit
-// sets first, so that all population loads of a cell are independent, and
-// every load comes before any store (the compiler cannot know that the 19
-// planes of lam_yp are distinct).
+// ones beside it.  Every row has face cells, so they take the common path.  The
+// destinations' flags are turned into bit sets first, so that all population
+// loads of a cell are independent, and every load comes before any store (the
+// compiler cannot know that the 19 planes of lam_yp are distinct).  128x64x48:
+// 41 us; 60 with a serial loop over a warp's face cells, 56 on 32-cell rows
+// with loads and stores plane by plane.
 __global__ void __launch_bounds__(256, 3) k_adj_stream(Dims d, CellDecode dec,
                                                        float* __restrict__ lam_yp,
                                                        const float* __restrict__ lam_xp,
@@ -202,7 +194,7 @@ __global__ void __launch_bounds__(128) k_adj_collide(
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < cnt; t += gridDim.x * blockDim.x) {
         const int c = tape_cells[t];
         int i, j, k;
-        cell_ijk(d, c, i, j, k);
+        d.ijk(c, i, j, k);
         float f[19];
 #pragma unroll
         for (int q = 0; q < 19; ++q) f[q] = tape_f[(int64_t)q * tape_cap + t];

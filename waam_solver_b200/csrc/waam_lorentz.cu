@@ -196,8 +196,8 @@ bool quads_ok(const Dims& d, const P*... p) {
 // A warp's share of the writing kernels: 32 consecutive k of V neighbouring
 // columns, so that it stays within one material (metal below, gas above) and
 // skips the arithmetic its cells do not need, while every thread still writes
-// 16 bytes (four columns' 128 cells in a row made every warp hold metal:
-// k_elec_J 152 us on 512x256x160 instead of 125 with one cell per thread).
+// 16 bytes (with four columns' 128 cells in a row every warp holds metal:
+// k_elec_J beside a step's pending stream 152 us on 512x256x160, 114 so).
 struct RowGrid {
     FastDiv by_kt, by_ny;
     int kt, ny, nz, ncol;
@@ -271,8 +271,9 @@ __global__ void __launch_bounds__(kTileK* kTileJ)
     }
 }
 
-// Pass 2: bound by the 4 bytes a cell it writes (512x256x160: 71 -> 51 us;
-// pass 1 57 -> 42).
+// Pass 2: bound by the exponential and the division of each cell in the slab
+// (84 % of the SMs' issue slots at 6 % of the DRAM rate; pass 1 the same).
+// 512x256x160, alone: 51 us, one cell per thread 71; pass 1 40 and 57.
 template <int V>
 __global__ void __launch_bounds__(kThreads)
     k_elec_source_fused_write(RowGrid g, float* src, float arc_i, float arc_j, float arc_k,
@@ -444,8 +445,9 @@ inline int64_t counts_total_len(int64_t nb) {
 
 // sigma, the fixed-cell mask and one live bit per cell.  Bound by memory: the
 // flags and the mask are read, sigma is written everywhere; f_l is read only
-// where a group of cells holds metal (512x256x160: 152 us with one cell per
-// thread and a block vote, 50 now).  V cells per thread (see load_cells); the
+// where a group of cells holds metal (512x256x160, alone: 46 us at 57 % of the
+// DRAM rate, 130 with one cell per thread and a block vote; beside a step's
+// pending stream 50 and 152).  V cells per thread (see load_cells); the
 // grid covers whole units, whose bits beyond the grid are 0.
 template <int V>
 __global__ void __launch_bounds__(kThreads)
@@ -699,8 +701,9 @@ __global__ void __launch_bounds__(kTileK* kTileJ)
     }
 }
 
-// kernels.py:1358-1383 elec_compute_J.  Bound by the 12 bytes a cell it writes
-// (most cells are gas and take zeros): 512x256x160 125 -> 114 us.
+// kernels.py:1358-1383 elec_compute_J.  Bound by latency: 58 registers keep 31 %
+// of the warps active, at half the DRAM rate.  512x256x160, alone: 94 us, with
+// one cell per thread 116 (beside a step's pending stream 114 and 125).
 template <int V>
 __global__ void __launch_bounds__(kThreads)
     k_elec_J(Dims d, RowGrid g, float* __restrict__ Jx, float* __restrict__ Jy,
@@ -863,9 +866,9 @@ __global__ void __launch_bounds__(256) k_elec_prefix(float* bins, int n_bins, in
 
 // kernels.py:1438-1475 elec_B_axisymmetric: V cells of a column per thread,
 // which share its radius, bin and r * dx; each cell takes the reference's
-// three divisions in its order.  Bound by those divisions where current flows
-// (512x256x160: 118 us, 127 with a warp per column), else by the 12 bytes a
-// cell it writes.
+// three divisions in its order.  Bound by those divisions (81 % of the SMs'
+// issue slots at 14 % of the DRAM rate).  512x256x160, alone: 106 us, 112 with
+// a warp per column (beside a step's pending stream 118 and 127).
 template <int V>
 __global__ void __launch_bounds__(kThreads)
     k_elec_B_cols(RowGrid g, float* __restrict__ Bx, float* __restrict__ By,

@@ -57,8 +57,9 @@ bool workspace_ok(void* ws, size_t bytes, int64_t n) {
 }
 
 // ---------------------------------------------------------------------------
-// Deterministic grid reduction: every block writes a double partial; the last
-// block to finish sums the partials in index order.
+// Deterministic grid reduction: every block writes a double partial; in the
+// last block to finish every thread adds a fixed strided share of them, then
+// the tree of block_sum: the order never changes.
 // ---------------------------------------------------------------------------
 __device__ double block_sum(double v) {
     __shared__ double sh[kThreads / 32];
@@ -85,8 +86,7 @@ __device__ bool finish_reduction(Workspace ws, double part, double& total) {
     __syncthreads();
     if (!last) return false;
     __threadfence();
-    // a fixed strided share of the partials per thread, then the fixed tree
-    // (one thread adding them all took 10 of the arc sum's 21 us)
+    // (one thread adding them all would take 10 us)
     double t = 0.0;
     for (unsigned b = threadIdx.x; b < gridDim.x; b += kThreads) t += __ldcg(ws.partials + b);
     t = block_sum(t);
@@ -517,11 +517,12 @@ __global__ void k_clamp_force(float* Fx, float* Fy, float* Fz, const int32_t* fl
     }
 }
 
-// One cell per thread.  Bound by memory on an all-fluid grid (228 bytes a
-// cell) and by latency on a melt pool's few active cells; left to itself the
-// compiler overlapped grid-stride iterations in 168 registers (one block of
-// 256 per SM).  Blocks of 128 at 64 registers keep 32 warps per SM: SRT on
-// 192x96x66 all fluid 94 -> 50 us, MRT on 101x61x43 17.5 -> 9.1 us.
+// One cell per thread.  188 bytes a fluid cell (19 populations in and out, 3
+// forces, f_l, the flag, density and velocity): SRT on 192x96x66 all fluid 50
+// us = 4.6 TB/s, 0.7 of the measured copy rate; with 32 warps per SM at 64
+// registers the rest is latency, and so is a melt pool's few active cells.
+// Left to itself the compiler overlaps grid-stride iterations in 168 registers
+// (one block of 256 per SM): 94 us; MRT on 101x61x43 17.5 us against 9.1.
 constexpr int kCollideThreads = 128;
 template <int KIND>
 __global__ void __launch_bounds__(kCollideThreads, 8)
@@ -1153,8 +1154,8 @@ int waam_collide_mrt(const float* f_src, float* f_dst, float* rho, float* ux, fl
     REQUIRE(f_src && f_dst && rho && ux && uy && uz && Fx && Fy && Fz && f_l && flags,
             "collide_mrt: null field");
     REQUIRE(f_src != f_dst, "collide_mrt: f_src must not alias f_dst");
-    COLLIDE(k_collide<0>, n, stream, f_src, f_dst, rho, ux, uy, uz, Fx, Fy, Fz, f_l, flags, n, omega_s,
-       omega_b, C_darcy, nullptr);
+    COLLIDE(k_collide<0>, n, stream, f_src, f_dst, rho, ux, uy, uz, Fx, Fy, Fz, f_l, flags, n,
+            omega_s, omega_b, C_darcy, nullptr);
 }
 
 int waam_collide_srt(const float* f_src, float* f_dst, float* rho, float* ux, float* uy, float* uz,
@@ -1163,8 +1164,8 @@ int waam_collide_srt(const float* f_src, float* f_dst, float* rho, float* ux, fl
     REQUIRE(f_src && f_dst && rho && ux && uy && uz && Fx && Fy && Fz && f_l && flags,
             "collide_srt: null field");
     REQUIRE(f_src != f_dst, "collide_srt: f_src must not alias f_dst");
-    COLLIDE(k_collide<1>, n, stream, f_src, f_dst, rho, ux, uy, uz, Fx, Fy, Fz, f_l, flags, n, omega,
-       0.0f, C_darcy, nullptr);
+    COLLIDE(k_collide<1>, n, stream, f_src, f_dst, rho, ux, uy, uz, Fx, Fy, Fz, f_l, flags, n,
+            omega, 0.0f, C_darcy, nullptr);
 }
 
 int waam_clamp_velocity_mach(float* ux, float* uy, float* uz, const int32_t* flags, int64_t n,
@@ -1297,8 +1298,8 @@ int waam_collide_srt_variable_tau(const float* f_src, float* f_dst, float* rho, 
     REQUIRE(f_src && f_dst && rho && ux && uy && uz && Fx && Fy && Fz && f_l && flags && tau_f,
             "collide_srt_variable_tau: null field");
     REQUIRE(f_src != f_dst, "collide_srt_variable_tau: f_src must not alias f_dst");
-    COLLIDE(k_collide<1>, n, stream, f_src, f_dst, rho, ux, uy, uz, Fx, Fy, Fz, f_l, flags, n, 0.0f,
-       0.0f, C_darcy, tau_f);
+    COLLIDE(k_collide<1>, n, stream, f_src, f_dst, rho, ux, uy, uz, Fx, Fy, Fz, f_l, flags, n,
+            0.0f, 0.0f, C_darcy, tau_f);
 }
 
 int waam_remelt_hot_solid(float* T, float* H, float* f_l, float* phi, int32_t* flags,
