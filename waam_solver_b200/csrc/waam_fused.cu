@@ -11,6 +11,7 @@
 // Cell kernels use 32x8 (k, j) tiles with one grid z-slice per i, so the cell
 // coordinates come from the launch geometry without integer division, and
 // consecutive lanes touch consecutive k (coalesced, k is the fastest axis).
+#include <algorithm>
 #include <cmath>
 #include <mutex>
 
@@ -690,18 +691,14 @@ __device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
 // tile_part (k_classify_tiles zeroes the quiet tiles' slots); the last block
 // adds all slots in tile order, so the total does not depend on the list's
 // order.  The surface query's arc k comes from k_classify_tiles.  A block
-// takes kArcBatch listed tiles at a time: their loads are all issued first --
-// the first batch's before the tables are built -- and their block sums share
-// one barrier.  Latency decides: the last block's sum of the slots, a chain of
+// takes kArcBatch listed tiles at a time, gridDim.x apart (so that a short list
+// reaches every block): their loads are all issued first -- the first batch's
+// before the tables are built -- and their block sums share one barrier.  Latency decides: the last block's sum of the slots, a chain of
 // four loads at a time, was half of the kernel on 512x256x160 (81,920 slots).
-// A short list goes to as many blocks as get kArcShare tiles each, one per SM
-// at least: further blocks wait for registers of the collision and the stream
-// beside them, and the sum ends with the last.  A step of 116x58x43 (about 950
-// tiles), 100x50x50 (700) and 128x64x48 (1050): 64.6, 52.7 and 69.6 us; on all
-// 592 blocks 66.0, 56.2 and 69.7; with five tiles each 64.0, 53.2 and 70.6.
+// The grid (arc_norm_blocks) is no larger than the grid of tiles can use: every
+// block, idle or not, waits for registers beside the collision and the stream,
+// and the sum ends with the last.
 constexpr int kArcBatch = 8;
-constexpr int kArcShare = 3;
-constexpr int kArcMinBlocks = 148;
 __global__ void __launch_bounds__(256, 4) k_arc_norm_list(Dims d, const int32_t* __restrict__ flags,
                                                        const float* __restrict__ f_l,
                                                        ArcParams p, float* scalars,
@@ -719,13 +716,12 @@ __global__ void __launch_bounds__(256, 4) k_arc_norm_list(Dims d, const int32_t*
     const int cnt = imin(list[0], tiles);
     const bool table = d.nz <= kArcTableMax;
     const bool axes = d.nx + d.ny + d.nz <= kArcAxisMax;
-    const int busy = imin((int)gridDim.x, imax(kArcMinBlocks, (cnt + kArcShare - 1) / kArcShare));
     int ent[kU], fg[kU], ck[kU];
     float fl[kU];
     auto load = [&](int e0) {
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
-            const int e = e0 + u * busy;
+            const int e = e0 + u * (int)gridDim.x;
             ent[u] = e < cnt ? list[1 + e] : -1;
         }
 #pragma unroll
@@ -737,7 +733,7 @@ __global__ void __launch_bounds__(256, 4) k_arc_norm_list(Dims d, const int32_t*
             ck[u] = k;
         }
     };
-    int e0 = (int)blockIdx.x < busy ? (int)blockIdx.x : cnt;
+    int e0 = blockIdx.x;
     if (e0 < cnt) {
         load(e0);
         p.arc_k = scalars[kScalarArcK] + arc_k_offset;
@@ -813,7 +809,7 @@ __global__ void __launch_bounds__(256, 4) k_arc_norm_list(Dims d, const int32_t*
             for (int w = 0; w < kWarps; ++w) sum += s_part[tid][w];
             tile_part[tile_index(d, mine)] = sum;
         }
-        e0 += kU * busy;
+        e0 += kU * (int)gridDim.x;
         if (e0 < cnt) load(e0);
         __syncthreads();
     }
@@ -1814,6 +1810,15 @@ constexpr int kTileListBlocks = 148 * 6;   // persistent grid of the work-list k
 // 19.6 us instead of 15.0 beside the collision, 512x256x160 68.6 instead of 48.2)
 constexpr int kInjectBlocks = 148 * 5;
 
+// The weight sum's grid: a block per eight tiles of the grid (a third to a half
+// of them are listed), one per SM at least.  A step of 100x50x50 (1,400 tiles,
+// 175 blocks) takes 50.4 us, with 592 blocks 56.3; 116x58x43 (232 blocks) 64.2
+// and 66.2; 128x64x48 (256 blocks) 71.2 and 71.0, with 148 blocks 74.1.
+static int arc_norm_blocks(int64_t n_tiles) {
+    const int64_t b = (n_tiles + 7) / 8;
+    return (int)std::min<int64_t>(n_tiles, std::min<int64_t>(kTileRedBlocks, std::max<int64_t>(b, 148)));
+}
+
 static VarPhase var_phase(const WaamStepParams* p) {
     return VarPhase{p->H_sol_t, p->H_liq_t, p->L_rho, p->Ts, p->Tl, p->T_cap};
 }
@@ -1928,11 +1933,9 @@ int waam_step_pre(const WaamFields* f, const WaamStepParams* p, void* workspace,
     ArcParams a = arc_params(p);
     float Qe_dt = p->Q_w * p->eta * p->dt;
     float* shape = reinterpret_cast<float*>(static_cast<char*>(workspace) + ws_shape_offset(d.n()));
-    const int tiles = (int)tile_grid(d).x * (int)tile_grid(d).y * d.nx;
-    const int blocks = tiles < kTileRedBlocks ? tiles : kTileRedBlocks;
     PhaseParams ph = make_phase(p->cp_rho, p->L_rho, p->Ts, p->Tl, p->T_cap, p->cap_enabled);
     if (tl) {
-        k_arc_norm_list<<<blocks, tile_block(), 0, s>>>(
+        k_arc_norm_list<<<arc_norm_blocks(n_tiles), tile_block(), 0, s>>>(
             d, f->flags, f->f_l, a, f->step_scalars, p->arc_k_offset, Qe_dt, p->dx3, ws, shape,
             f->tile_list, f->tile_part, (int)n_tiles);
         int e = check_launch("k_arc_norm_list");
@@ -1944,6 +1947,7 @@ int waam_step_pre(const WaamFields* f, const WaamStepParams* p, void* workspace,
             (int)n_tiles);
         return check_launch("k_arc_inject_list");
     }
+    const int blocks = (int)(n_tiles < kTileRedBlocks ? n_tiles : kTileRedBlocks);
     k_arc_norm_tiles<<<blocks, tile_block(), 0, s>>>(
         d, f->flags, f->f_l, f->phi, p->nz_solid, a, f->step_scalars, p->arc_k_offset, Qe_dt,
         p->dx3, ws, shape);
