@@ -30,7 +30,7 @@ def rows(monkeypatch):
 
     monkeypatch.setattr(adjoint, "_call", call)
     monkeypatch.setattr(adjoint, "_stream", lambda: 0)
-    monkeypatch.setattr(adjoint, "_on_current_device", lambda t: True, raising=False)
+    monkeypatch.setattr(adjoint, "_device", lambda: -1, raising=False)     # the CPU's
     return sent
 
 

@@ -50,33 +50,36 @@ def _ptr(t):
 _stream = _native.stream_handle
 
 
-def _on_current_device(t):
-    return t.is_cuda and t.device.index == torch.cuda.current_device()
+def _device():
+    return torch.cuda.current_device()
 
 
-def _raw_copy(dst, src):
-    """Whether dst.copy_(src) is a copy of src's bytes that the kernel can make."""
-    return (dst.shape == src.shape and dst.dtype == src.dtype and dst.device == src.device and
-            dst.is_contiguous() and src.is_contiguous() and
-            src.numel() * src.element_size() % 4 == 0 and _on_current_device(src))
+def _raw_bytes(dst, src, device):
+    """Size of the copy where dst.copy_(src) is one of src's bytes, in whole words
+    on the current device, else None."""
+    size = src.nbytes
+    if (size % 4 == 0 and dst.nbytes == size and dst.dtype is src.dtype and
+            dst.get_device() == device and src.get_device() == device and
+            dst.shape == src.shape and dst.is_contiguous() and src.is_contiguous()):
+        return size
+    return None
 
 
 def _copy_planes(pairs):
     """dst.copy_(src) for every (dst, src) pair, the plain copies in one launch
     (per 32 of them); the others convert, or raise, as copy_ does, before any
     plain one is made."""
+    device = _device()
     raw = []
     for dst, src in pairs:
-        if _raw_copy(dst, src):
-            raw.append((dst, src))
-        else:
+        size = _raw_bytes(dst, src, device)
+        if size is None:
             dst.copy_(src)
+        else:
+            raw.append((dst.data_ptr(), src.data_ptr(), size))
     for s0 in range(0, len(raw), _native.MAX_COPY_PLANES):
         part = raw[s0:s0 + _native.MAX_COPY_PLANES]
-        table = (_native.WaamCopyPlane * len(part))()
-        for row, (dst, src) in zip(table, part):
-            row.dst, row.src = dst.data_ptr(), src.data_ptr()
-            row.bytes = src.numel() * src.element_size()
+        table = (_native.WaamCopyPlane * len(part))(*part)
         _call("waam_copy_planes", ctypes.byref(table), len(part), _stream())
 
 
@@ -295,7 +298,7 @@ class AdjointProblem:
         self.hist = torch.zeros((self.N, max(2 * P, 2)), dtype=torch.float32, device=g.device)
         self.scal = torch.zeros((self.N, 16), dtype=torch.float32, device=g.device)
         self.checkpoints = {}
-        if not _raw_copy(self.scal[0], g.step_scalars):
+        if _raw_bytes(self.scal[0], g.step_scalars, _device()) is None:
             raise WaamError("the step scalars are not %d floats" % self.scal.shape[1])
         scal_row = 4 * self.scal.shape[1]
         row = _native.WaamCopyPlane(bytes=scal_row)
