@@ -61,6 +61,15 @@ def test_other_types_and_orders_go_through_copy(rows):
     assert torch.equal(a, x.float()) and torch.equal(b, y) and torch.equal(c, z)
 
 
+def test_copies_alike_are_checked_at_their_source(rows):
+    src = [torch.rand(3, 5), torch.rand(4, 6).t(), torch.arange(5, dtype=torch.uint8)]
+    dst = [torch.empty_like(t) for t in src]
+    adjoint._copy_planes(zip(dst, src), alike=True)
+    assert len(rows) == 1
+    rows.copy_all()
+    assert all(torch.equal(a, b) for a, b in zip(dst, src))
+
+
 def _grid(n=24, **other):
     f = lambda: torch.rand(n)  # noqa: E731
     g = types.SimpleNamespace(n_cells=n, device=torch.device("cpu"), H=f(), T=f(), H_next=f(),

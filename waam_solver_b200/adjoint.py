@@ -54,25 +54,25 @@ def _device():
     return torch.cuda.current_device()
 
 
-def _raw_bytes(dst, src, device):
+def _raw_bytes(dst, src, device, alike=False):
     """Size of the copy where dst.copy_(src) is one of src's bytes, in whole words
-    on the current device, else None."""
+    on the current device, else None.  ``alike``: dst is torch.empty_like(src)."""
     size = src.nbytes
-    if (size % 4 == 0 and dst.nbytes == size and dst.dtype is src.dtype and
-            dst.get_device() == device and src.get_device() == device and
-            dst.shape == src.shape and dst.is_contiguous() and src.is_contiguous()):
+    if (size % 4 == 0 and src.is_contiguous() and src.get_device() == device and
+            (alike or (dst.get_device() == device and dst.dtype is src.dtype and
+                       dst.is_contiguous() and dst.shape == src.shape))):
         return size
     return None
 
 
-def _copy_planes(pairs):
+def _copy_planes(pairs, alike=False):
     """dst.copy_(src) for every (dst, src) pair, the plain copies in one launch
     (per 32 of them); the others convert, or raise, as copy_ does, before any
     plain one is made."""
     device = _device()
     raw = []
     for dst, src in pairs:
-        size = _raw_bytes(dst, src, device)
+        size = _raw_bytes(dst, src, device, alike)
         if size is None:
             dst.copy_(src)
         else:
@@ -95,7 +95,7 @@ class _Checkpoint:
         g.flush_stream()
         state = _state_tensors(g)
         self.t = [torch.empty_like(t) for t in state]
-        _copy_planes(list(zip(self.t, state)))
+        _copy_planes(zip(self.t, state), alike=True)
         self.g_host = (g._read_buf is g.f_a, g._cur, getattr(g, "_forces_dirty", True),
                        getattr(g, "_tracers_live", False))
         self.host = {k: getattr(tw, k) for k in _HOST}
@@ -106,7 +106,7 @@ class _Checkpoint:
         g._collide_pending = False
         g._lag_pending = False
         g._tiles_valid = False          # the quiet-tile history is not the checkpoint's
-        _copy_planes(list(zip(_state_tensors(g), self.t)))
+        _copy_planes(zip(_state_tensors(g), self.t))
         read_a, g._cur, g._forces_dirty, live = self.g_host
         g._read_buf, g._write_buf = (g.f_a, g.f_b) if read_a else (g.f_b, g.f_a)
         if live != getattr(g, "_tracers_live", False):
