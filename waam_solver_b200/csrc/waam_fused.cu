@@ -282,8 +282,8 @@ __device__ __forceinline__ bool is_active(int flag) { return flag == FLUID || fl
 // 192x96x66 all fluid: 44.8 us against 64 with a flag load per population (and
 // 32-cell rows, a third of whose lanes nz = 66 left idle).  With the other
 // form, whose mending is a tail that nothing hides, steps with the remelt tail
-// take 3 % longer on 64x32x32 and 80x48x32, 1 % on 256x128x96 (and 0.5 % less
-// there with 2-byte elements).
+// take 3 % longer on 64x32x32 and 80x48x32, 1 % on 256x128x96 (with 2-byte
+// elements, on four blocks per SM since 48 registers spill, 4 % and the same).
 // Else, beside the next step's stages: few cells bounce (the melt surface), so
 // they are mended after the stores and the kernel keeps the registers of a
 // plain copy.  What a 256x128x96 step waits for is its end: with the votes'
@@ -295,7 +295,7 @@ __device__ __forceinline__ bool is_active(int flag) { return flag == FLUID || fl
 // of WaamStepParams.hold_stream).
 constexpr int kStreamThreads = 256;
 template <typename T, bool VOTE>
-__global__ void __launch_bounds__(kStreamThreads, VOTE ? 5 : 6)
+__global__ void __launch_bounds__(kStreamThreads, !VOTE ? 6 : sizeof(T) == 4 ? 5 : 4)
     k_stream(const __grid_constant__ StreamGrid g, const __grid_constant__ StreamPtrs<T> P,
              const int32_t* __restrict__ flags, const int32_t* __restrict__ next_flags) {
     const unsigned at = blockIdx.x * kStreamThreads + threadIdx.x;
